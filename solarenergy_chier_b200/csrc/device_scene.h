@@ -24,7 +24,7 @@ struct DevGrid {
                         // for k = lattice x, normal, lattice z, then (x0, 1/px, z0, 1/pz)
   const int4* hsub;     // (first sub-heliostat id, count, lattice rows, lattice columns) per grid-local heliostat
   const float4* subv;   // 3 float4 per sub-heliostat: A.xyz AB.x | AB.yz AC.xy | AC.z
-  // Per sub-heliostat, for its facets' block walks (qm::block_candidates):
+  // Per sub-heliostat, for its facets' block walks (qm::warp_candidates):
   // 1 = skipped (nothing can be hit), k + 1 = only the k <= kMaxCandidates
   // heliostats in sub_cand[kMaxCandidates * sub ...] can be hit (a ray
   // meeting none of their padded boxes skips the walk), 0 = walk.
@@ -73,7 +73,7 @@ struct DevTask {
   const float4* samples;        // sun-shape pool already turned into world space by this task's sun
   const float4* perturbations;  // slope-error pool (local frame of the facet normal)
   int pool_size;                // P = groups x lights per group
-  // Shadow walks of this heliostat's rays (qm::cone_candidates around the
+  // Shadow walks of this heliostat's rays (qm::warp_candidates around the
   // sun-shape cone): 1 = skipped (nothing can shadow them), k + 1 = only the
   // k listed heliostats can (a ray meeting none of their padded boxes skips
   // its walk), 0 = walk.

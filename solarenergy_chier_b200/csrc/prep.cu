@@ -69,78 +69,86 @@ __device__ __forceinline__ int candidate_code(int k) {
   return k == 0 ? 1 : (k > 0 && k <= kMaxCandidates ? k + 1 : 0);
 }
 
-// Walk codes of the prepared tasks: thread j handles task j / (1 + max_sub),
+// Code and candidate list of one cone (state: make_cone's result), by a whole
+// warp; `cand` holds kMaxCandidates entries.
+__device__ __forceinline__ int warp_code(const ShadowGrid& view, int own, int state, const Cone& cone, int* cand) {
+  if (state < 0) return 0;
+  if (state == 0) return 1;
+  int found;
+  const int k = warp_candidates(view, own, cone, kMaxCandidates, found);
+  if (k <= kMaxCandidates && (int)(threadIdx.x & 31) < k) cand[threadIdx.x & 31] = found;
+  return candidate_code(k);
+}
+
+__device__ __forceinline__ float3 sub_normal(const DevTask& T, int s) {
+  Frame hf;
+  hf.u = T.fu;
+  hf.n = T.fn;
+  hf.v = T.fv;
+  hf.identity = T.frame_identity != 0;
+  return T.type == 1 ? qs::to_world(hf, T.local_normals[s]) : T.normal;
+}
+
+// Walk codes of the prepared tasks: warp j handles task j / (1 + max_sub),
 // slot j % (1 + max_sub): slot 0 its shadow walks, slot 1 + s the block
 // walks of its sub-heliostat s (each a capsule enumeration of its own).
 __global__ void shadow_kernel(const PrepItem* items, int n, int max_sub, DevTask* tasks, const DevGrid* grids) {
-  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long j = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
   const int i = (int)(j / (1 + max_sub)), slot = (int)(j % (1 + max_sub));
   if (i >= n) return;
   const PrepItem& it = items[i];
   DevTask& T = tasks[it.task];
   const DevGrid& G = grids[T.grid];
   const ShadowGrid view{G.pos, G.interval, G.cells, G.bound, G.cell_range, G.entries};
+  Cone cone;
   if (slot == 0) {
-    T.shadow_free = candidate_code(it.shadow_tan >= 0.0f ? shadow_candidates(view, T.own, it.shadow_axis,
-                                                                            it.shadow_tan, T.shadow_cand,
-                                                                            kMaxCandidates)
-                                                         : -1);
+    const int state = it.shadow_tan >= 0.0f ? shadow_cone(view, T.own, it.shadow_axis, it.shadow_tan, cone) : -1;
+    const int code = warp_code(view, T.own, state, cone, T.shadow_cand);
+    if (lane == 0) T.shadow_free = code;
     return;
   }
   const int s = slot - 1;
   if (s >= it.num_sub) return;
-  Frame hf;
-  hf.u = T.fu;
-  hf.n = T.fn;
-  hf.v = T.fv;
-  hf.identity = T.frame_identity != 0;
-  const float3 nrm = T.type == 1 ? qs::to_world(hf, T.local_normals[s]) : T.normal;
-  sub_frames(T, s, it.sub_frames + 6 * s);
-  const int k = it.block_theta >= 0.0f ? block_candidates(view, T.own, it.verts + 3 * s, it.sun_dir, nrm,
-                                                         it.block_theta, it.sub_cand + kMaxCandidates * s,
-                                                         kMaxCandidates)
-                                       : -1;
-  it.sub_free[s] = candidate_code(k);
+  if (lane == 0) sub_frames(T, s, it.sub_frames + 6 * s);
+  const int state = it.block_theta >= 0.0f
+                        ? block_cone(view, it.verts + 3 * s, it.sun_dir, sub_normal(T, s), it.block_theta, cone)
+                        : -1;
+  const int code = warp_code(view, T.own, state, cone, it.sub_cand + kMaxCandidates * s);
+  if (lane == 0) it.sub_free[s] = code;
 }
 
 // Walk codes of a plain scene's heliostats (its task templates), with the
-// same thread layout as shadow_kernel; the sub-heliostat parallelograms are
+// same warp layout as shadow_kernel; the sub-heliostat parallelograms are
 // read back from the traversal form (A, B - A, C - A) -- the tests are
 // conservative far above that rounding.
 __global__ void walk_flags_kernel(WalkFlagParams p) {
-  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const long long j = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int lane = threadIdx.x & 31;
   const int i = (int)(j / (1 + p.max_sub)), slot = (int)(j % (1 + p.max_sub));
   if (i >= p.n) return;
   const DevTask& T = p.tasks[i];
   const DevGrid& G = p.grids[T.grid];
   const ShadowGrid view{G.pos, G.interval, G.cells, G.bound, G.cell_range, G.entries};
+  Cone cone;
   if (slot == 0) {
-    p.shadow_out[i] = candidate_code(p.sun_tan >= 0.0f ? shadow_candidates(view, T.own, p.sun_axis, p.sun_tan,
-                                                                           p.shadow_cand_out + kMaxCandidates * i,
-                                                                           kMaxCandidates)
-                                                        : -1);
+    const int state = p.sun_tan >= 0.0f ? shadow_cone(view, T.own, p.sun_axis, p.sun_tan, cone) : -1;
+    const int code = warp_code(view, T.own, state, cone, p.shadow_cand_out + kMaxCandidates * i);
+    if (lane == 0) p.shadow_out[i] = code;
     return;
   }
   const int s = slot - 1;
   const int4 hs = G.hsub[T.own];
   if (s >= hs.y) return;
-  Frame hf;
-  hf.u = T.fu;
-  hf.n = T.fn;
-  hf.v = T.fv;
-  hf.identity = T.frame_identity != 0;
-  int* sub_free = const_cast<int*>(G.sub_free);
-  int* sub_cand = const_cast<int*>(G.sub_cand);
-  sub_frames(T, s, const_cast<float4*>(G.sub_frames) + 6 * (hs.x + s));
+  if (lane == 0) sub_frames(T, s, const_cast<float4*>(G.sub_frames) + 6 * (hs.x + s));
   const float4* q = G.subv + 3 * (hs.x + s);
   const float3 A = make_float3(q[0].x, q[0].y, q[0].z);
   const float3 bac[3] = {make_float3(A.x + q[0].w, A.y + q[1].x, A.z + q[1].y), A,
                          make_float3(A.x + q[1].z, A.y + q[1].w, A.z + q[2].x)};
-  const float3 nrm = T.type == 1 ? qs::to_world(hf, T.local_normals[s]) : T.normal;
-  const int k = p.block_theta >= 0.0f ? block_candidates(view, T.own, bac, p.sun_dir, nrm, p.block_theta,
-                                                        sub_cand + kMaxCandidates * (hs.x + s), kMaxCandidates)
-                                      : -1;
-  sub_free[hs.x + s] = candidate_code(k);
+  const int state =
+      p.block_theta >= 0.0f ? block_cone(view, bac, p.sun_dir, sub_normal(T, s), p.block_theta, cone) : -1;
+  const int code = warp_code(view, T.own, state, cone, const_cast<int*>(G.sub_cand) + kMaxCandidates * (hs.x + s));
+  if (lane == 0) const_cast<int*>(G.sub_free)[hs.x + s] = code;
 }
 
 // Pool of instance blockIdx.y turned by that instance's sun frame.
@@ -173,16 +181,20 @@ cudaError_t launch_shadow_flags(const PrepItem* items, int n, int max_sub, DevTa
                                 cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
   if (max_sub < 0) return cudaErrorInvalidValue;
-  const long long threads = (long long)n * (1 + max_sub);
-  shadow_kernel<<<(unsigned)((threads + 63) / 64), 64, 0, stream>>>(items, n, max_sub, tasks, grids);
+  const long long warps = (long long)n * (1 + max_sub);
+  const long long blocks = (warps + 3) / 4;  // four warps a block, a warp per cone
+  if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+  shadow_kernel<<<(unsigned)blocks, 128, 0, stream>>>(items, n, max_sub, tasks, grids);
   return cudaGetLastError();
 }
 
 cudaError_t launch_walk_flags(const WalkFlagParams& p, cudaStream_t stream) {
   if (p.n <= 0) return cudaSuccess;
   if (p.max_sub < 0) return cudaErrorInvalidValue;
-  const long long threads = (long long)p.n * (1 + p.max_sub);
-  walk_flags_kernel<<<(unsigned)((threads + 63) / 64), 64, 0, stream>>>(p);
+  const long long warps = (long long)p.n * (1 + p.max_sub);
+  const long long blocks = (warps + 3) / 4;
+  if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+  walk_flags_kernel<<<(unsigned)blocks, 128, 0, stream>>>(p);
   return cudaGetLastError();
 }
 

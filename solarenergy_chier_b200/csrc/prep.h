@@ -64,7 +64,7 @@ cudaError_t launch_walk_flags(const WalkFlagParams& p, cudaStream_t stream);
 cudaError_t launch_prep(const PrepItem* items, int n, DevTask* tasks, cudaStream_t stream);
 // Shadow-free flags of the prepared tasks; grids: the tasks' grids with their
 // prepared traversal records.  Run after launch_prep.
-// max_sub: the most sub-heliostats of any item (one thread per heliostat and
+// max_sub: the most sub-heliostats of any item (one warp per heliostat and
 // per sub-heliostat).
 cudaError_t launch_shadow_flags(const PrepItem* items, int n, int max_sub, DevTask* tasks, const DevGrid* grids,
                                 cudaStream_t stream);

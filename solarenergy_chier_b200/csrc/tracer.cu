@@ -560,7 +560,7 @@ __global__ void __launch_bounds__(kThreads, QM_TRACE_MIN_BLOCKS) trace_kernel(QM
         win.o[wbase + lane] = make_float4(origin.x, origin.y, origin.z, __int_as_float(__ldg(T.offsets + fw)));
         // Pool offsets lie below 2^30; bit 31 carries the facet's
         // sub-heliostat block-free flag, and the frame word below its
-        // candidate blockers (qm::block_candidates): n.w = sub-heliostat << 4
+        // candidate blockers (qm::warp_candidates): n.w = sub-heliostat << 4
         // | candidates << 1 | frame identity.
         const int bcode = __ldg(G.sub_free + sub);
         const int free_bit = bcode == 1 ? (int)0x80000000 : 0;
@@ -582,7 +582,7 @@ __global__ void __launch_bounds__(kThreads, QM_TRACE_MIN_BLOCKS) trace_kernel(QM
       const float3 dir = xyz(__ldg(lds_ptr(win.samples[threadIdx.x >> 5]) + __float_as_int(win.o[slot].w) + lab));
       int32_t code;
       // Heliostats whose rays no other heliostat can shadow skip the shadow
-      // walk; where only a few listed heliostats can (qm::cone_candidates,
+      // walk; where only a few listed heliostats can (qm::warp_candidates,
       // decided per sun when the task is built), candidate_hit decides.
       const int sc = lds_int(win.shadow_free[threadIdx.x >> 5]);
       int shadowed = sc == 1 ? 0 : -1;  // -1: walk
@@ -609,7 +609,7 @@ __global__ void __launch_bounds__(kThreads, QM_TRACE_MIN_BLOCKS) trace_kernel(QM
         float3 rd = qx::normalize_unit(qx::reflect(neg(dir), n));
         // Facets of sub-heliostats no other heliostat can block skip the
         // block walk; where only a few listed heliostats can
-        // (qm::block_candidates, decided per sun with the pools),
+        // (qm::warp_candidates, decided per sun with the pools),
         // candidate_hit decides.
         int blocked = 0;
         if (g1 >= 0) {

@@ -57,3 +57,39 @@ def test_device_grid_build_equals_host(kind, tmp_path, cuda_device):
     s.clear_power()
     s.trace(ids)
     np.testing.assert_allclose(s.power()[0], before, rtol=1e-12, atol=0)
+
+
+@pytest.mark.parametrize("kind", ["small", "large", "uneven", "two", "huge"])
+def test_walk_codes_equal_a_sequential_enumeration(kind, tmp_path, cuda_device):
+    """The warps' candidate lists (csrc/shadow.h) against one sequential
+    enumeration per cone on the host (tests/walk_codes_main.cpp): the same code
+    for every heliostat and sub-heliostat, at a high and a low sun, with and
+    without a wide sun shape (cones from one cell to too many to enumerate).
+    Integers, so equal: host and device round the cones alike but for the
+    tangent and arc tangent of a cone's angle, against a 5 cm margin."""
+    import subprocess
+
+    from solarenergy_chier_b200 import build
+
+    f = fields(kind, tmp_path)
+    exe = tmp_path / "walk_codes"
+    r = subprocess.run(["g++", "-std=c++17", "-O2", "-ffp-contract=off", f"-I{build.CSRC}", f"-I{build.INCLUDE}",
+                        f"-I{build.CUDA_HOME / 'include'}", str(build.ROOT / "tests" / "walk_codes_main.cpp"),
+                        str(build.CSRC / "scene.cpp"), "-o", str(exe)], capture_output=True, text=True)
+    assert r.returncode == 0, r.stderr
+    s = q.Scene(f.scene, f.config, device=0, seed=3)
+    seen = set()
+    for half_angle in (0.00465, 0.05):
+        s.generate_sample_pool(5, q.SUNSHAPE_PILLBOX, half_angle)
+        dirs, pert = s.get_sample_pool()
+        tan = [np.max(np.hypot(p[:, 0].astype(np.float64), p[:, 2]) / p[:, 1]) for p in (dirs, pert)]
+        for sun in (synth.sun_direction(180.0, 60.0), synth.sun_direction(110.0, 15.0)):
+            s.set_sun(sun)
+            args = [repr(float(np.float32(v))) for v in sun] + [f"{tan[0]:.9g}", f"{np.arctan(tan[1]):.9g}"]
+            out = subprocess.run([str(exe), str(f.scene), str(f.config), *args], capture_output=True, text=True)
+            assert out.returncode == 0
+            got = np.concatenate([s.shadow_free()] + [s.block_free(g) for g in range(s.num_grids)])
+            want = np.array(out.stdout.split(), np.int32)
+            assert np.array_equal(got, want), f"{np.count_nonzero(got != want)} of {len(want)} codes differ"
+            seen |= set(np.unique(got).tolist())
+    print(kind, "codes seen", sorted(seen))
