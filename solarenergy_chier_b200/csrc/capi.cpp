@@ -1213,6 +1213,11 @@ int qmcrt_smooth(float* d_img, int width, int height, int radius, float ratio, v
     if (radius < 0 || radius > 64) invalid("radius must be in [0, 64]");
     if (!(ratio >= 0.0f && ratio < 0.5f)) invalid("trim ratio must be in [0, 0.5)");
     cudaStream_t st = static_cast<cudaStream_t>(stream);
+    const cudaError_t in_place = qm::launch_trimmed_mean_in_place(d_img, width, height, radius, ratio, st);
+    if (in_place != cudaErrorNotSupported) {
+      cuda_check(in_place, "trimmed mean");
+      return;
+    }
     const size_t bytes = (size_t)width * height * sizeof(float);
     void* copy = nullptr;
     alloc_gate("cudaMallocAsync");

@@ -258,6 +258,29 @@ def test_smoother_matches_oracle(small, shape, radius, ratio):
     assert np.array_equal(got, want)
 
 
+@pytest.mark.parametrize("shape,radius,ratio", [
+    ((8, 32), 2, 0.1), ((9, 33), 2, 0.1), ((7, 31), 2, 0.1),       # one tile, just past it, just short of it
+    ((40, 70), 1, 0.0), ((40, 70), 1, 0.45), ((300, 5), 4, 0.05),  # no trim; the largest 3x3 trim; narrower than a window
+    ((33, 65), 3, 0.31), ((33, 65), 3, 0.33), ((60, 90), 12, 0.025),  # 15 trimmed (registers), 16 (shared memory); wide
+    ((2100, 4096), 1, 0.17)])                                      # past the SMs' shared memory: smoothed from a copy
+def test_smoother_tile_and_trim_edges(shape, radius, ratio):
+    """The register kernel's tile edges, trims and both ways of holding the
+    image against the oracle: the same heaps and sums, so equal, infinite and
+    NaN pixels included."""
+    import torch
+
+    rng = np.random.default_rng(shape[1] + radius)
+    img = (rng.random(shape) * 100).astype(np.float32)
+    img[rng.random(shape) < 0.4] = 0
+    if shape == (60, 90):
+        img[20, 30], img[50, 80], img[5, 5] = np.inf, -np.inf, np.nan
+    want = oracle.smooth(img, radius, ratio)
+    t = torch.from_numpy(img).cuda()
+    q.smooth_device(t.data_ptr(), shape[1], shape[0], radius, ratio)
+    torch.cuda.synchronize()
+    assert np.array_equal(t.cpu().numpy(), want, equal_nan=True)
+
+
 def binned(img, k=8):
     h, w = img.shape
     h2, w2 = h // k * k, w // k * k
