@@ -106,7 +106,10 @@ void batch_prepare(qmcrt_batch* b, cudaStream_t st) {
 
 void batch_build_prefix(qmcrt_batch* b) {
   const long long nl = b->light_end - b->light_begin;
-  const long long chunk = chunk_rays_for(b->mode, b->shape, 0);
+  long long all_rays = 0;
+  for (const auto& t : b->tasks) all_rays += (long long)t.num_facets * nl;
+  b->chunk_iters = b->hit_record_chunks ? qm::kChunkIters : chunk_iters_for(b->mode, b->shape, 0, all_rays);
+  const long long chunk = 32LL * b->chunk_iters;
   std::vector<long long> prefix(b->tasks.size() + 1, 0);
   for (size_t i = 0; i < b->tasks.size(); ++i) {
     const long long rays = (long long)b->tasks[i].num_facets * nl;
@@ -135,9 +138,8 @@ cudaError_t batch_launch(qmcrt_batch* b, cudaStream_t st, int out, long long chu
   p.diag = b->d_diag.as<unsigned long long>();
   p.hit_bits = b->hit_bits;
   if (out == 0 || out == 2) p.chunk_power = b->d_chunk_power.as<double>();
-  // the prefix is laid out for the flux kernel's chunk size
-  if (chunk_rays_for(b->mode, b->shape, out) != chunk_rays_for(b->mode, b->shape, 0)) return cudaErrorInvalidValue;
-  return launch_trace_mode(b->mode, p, out, st, b->shape, out == 0 ? b->d_work.as<unsigned long long>() : nullptr);
+  return launch_trace_mode(b->mode, p, out, st, b->shape, b->chunk_iters,
+                           out == 0 ? b->d_work.as<unsigned long long>() : nullptr);
 }
 
 }  // namespace qrt
@@ -309,6 +311,7 @@ int qmcrt_batch_set_math_mode(qmcrt_batch* b, int mode) {
     batch_checked(b);
     if (mode < 0 || mode > 4) invalid("math mode must be 0, 1, 2, 3 or 4");
     b->mode = mode;
+    b->total_chunks = -1;  // a build's launch shape decides the chunks
     b->drop_graph();
   });
 }

@@ -30,6 +30,10 @@ struct qmcrt_batch {
   qrt::DBuf d_work;         // work counter of persistent flux launches
   int light_begin = 0, light_end = 0, max_lights = 0;
   long long total_chunks = -1;  // for the current light range; -1 = prefix not built
+  int chunk_iters = qm::kChunkIters;  // warp-chunk iterations of the prefix
+  // Bilinear-deposit and hit-bit launches share the prefix (a differentiable
+  // pair's batch): their buffers hold one word per iteration of kChunkIters.
+  bool hit_record_chunks = false;
   int mode = 0;                 // 0 production, 1 exact, 2 production at 64 registers, 3 approximate math
   int shape = 0;                // launch shape of the production build (qmcrt_batch_set_launch_shape)
   uint32_t* hit_bits = nullptr;  // output of bilinear-deposit launches (owned by the caller)

@@ -442,34 +442,51 @@ qm::TraceParams base_params(qmcrt_scene* s) {
 // deposits keep shape 0, whose chunk layout the other outputs share.
 struct LaunchShape {
   int threads, chunk_iters, persistent;
-  cudaError_t (*launch)(const qm::TraceParams&, int, cudaStream_t, unsigned long long*);
-  int (*chunk_rays)();
+  cudaError_t (*launch)(const qm::TraceParams&, int, cudaStream_t, unsigned long long*, int);
 };
 const LaunchShape kShapes[] = {
-    {32, 64, 0, qm::launch_trace_fast, qm::trace_chunk_rays_fast},
-    {32, 32, 0, qm::launch_trace_fast_c32, qm::trace_chunk_rays_fast_c32},
-    {32, 128, 0, qm::launch_trace_fast_c128, qm::trace_chunk_rays_fast_c128},
-    {64, 64, 0, qm::launch_trace_fast_t64, qm::trace_chunk_rays_fast_t64},
-    {256, 64, 0, qm::launch_trace_fast4, qm::trace_chunk_rays_fast4},
-    {32, 64, 1, qm::launch_trace_fast_ps, qm::trace_chunk_rays_fast_ps},
+    {32, 64, 0, qm::launch_trace_fast},
+    {32, 32, 0, qm::launch_trace_fast_c32},
+    {32, 128, 0, qm::launch_trace_fast_c128},
+    {64, 64, 0, qm::launch_trace_fast_t64},
+    {256, 64, 0, qm::launch_trace_fast4},
+    {32, 64, 1, qm::launch_trace_fast_ps},
 };
 constexpr int kNumShapes = sizeof(kShapes) / sizeof(kShapes[0]);
 
 int shape_for(int mode, int shape, int out) { return (mode == 0 && out == 0 && shape > 0 && shape < kNumShapes) ? shape : 0; }
 
-long long chunk_rays_for(int mode, int shape, int out) {
-  return kShapes[shape_for(mode, shape, out)].chunk_rays();
+// A warp runs its chunk's iterations one after another (about 0.9 us each), so
+// a launch takes at least a chunk's time however few rays it has, and its
+// last wave of chunks leaves slots idle for as long; a smaller chunk pays more
+// often for the task lookup, the facet window and the power sum.  Production
+// build, us at 8 / 16 / 64 iterations (148 SMs x 28 warps):
+//   one heliostat, 0.4 M rays 17 / 23 / 63, 1.6 M 40 / 39 / 66, 6.6 M 139 / 130 / 123;
+//   648 focus-flat, 3 M 107 / 128 / 247, 6 M 154 / 169 / 256, 24 M 495 / 480 / 560;
+//   50 flat, 41 M 750 / 753 / 774; 48 focus-flat, 58 M 864 / 842 / 848,
+//   115 M 1,576 / 1,524 / 1,504
+// (the exact build moves alike).  So 8 until 16 would make three waves, 64
+// from 64 M rays on.
+constexpr long long kWaveWarps = 148 * 28;
+constexpr long long kMediumLaunchRays = 3 * kWaveWarps * 32 * qm::kMediumChunkIters;  // 6.4 M
+constexpr long long kLargeLaunchRays = 64LL * 1000 * 1000;
+
+int chunk_iters_for(int mode, int shape, int out, long long rays) {
+  const int sh = shape_for(mode, shape, out);
+  if (sh == 0 && out == 0 && rays < kLargeLaunchRays)
+    return rays < kMediumLaunchRays ? qm::kSmallChunkIters : qm::kMediumChunkIters;
+  return kShapes[sh].chunk_iters;
 }
 
-cudaError_t launch_trace_mode(int mode, const qm::TraceParams& p, int out, cudaStream_t st, int shape,
+cudaError_t launch_trace_mode(int mode, const qm::TraceParams& p, int out, cudaStream_t st, int shape, int chunk_iters,
                               unsigned long long* work_counter) {
   cudaError_t e;
   switch (mode) {
-    case 1: e = qm::launch_trace_exact(p, out, st); break;
-    case 2: e = qm::launch_trace_fast4(p, out, st); break;
-    case 3: e = qm::launch_trace_approx(p, out, st); break;
-    case 4: e = qm::launch_trace_rx(p, out, st); break;
-    default: e = kShapes[shape_for(mode, shape, out)].launch(p, out, st, work_counter); break;
+    case 1: e = qm::launch_trace_exact(p, out, st, nullptr, chunk_iters); break;
+    case 2: e = qm::launch_trace_fast4(p, out, st, nullptr, chunk_iters); break;
+    case 3: e = qm::launch_trace_approx(p, out, st, nullptr, chunk_iters); break;
+    case 4: e = qm::launch_trace_rx(p, out, st, nullptr, chunk_iters); break;
+    default: e = kShapes[shape_for(mode, shape, out)].launch(p, out, st, work_counter, chunk_iters); break;
   }
   // flux and bilinear-deposit launches add their per-chunk power partials
   if (e == cudaSuccess && (out == 0 || out == 2) && p.chunk_power) e = qm::launch_power_reduce(p, st);
@@ -480,11 +497,6 @@ double* chunk_power_buffer(DBuf& buf, long long chunks) {
   const size_t need = (size_t)std::max<long long>(chunks, 1) * sizeof(double);
   if (buf.bytes < need) buf.alloc(need);
   return buf.as<double>();
-}
-
-cudaError_t run_trace(const qmcrt_scene* s, const qm::TraceParams& p, int out, cudaStream_t st,
-                      unsigned long long* work_counter) {
-  return launch_trace_mode(s->exact, p, out, st, s->shape, work_counter);
 }
 
 // Traces heliostats ids[0..n) over the scene's light range: out 0 adds their
@@ -502,7 +514,10 @@ long long trace_ids(qmcrt_scene* s, const int* ids, int n, cudaStream_t stream, 
   DeviceGuard guard(s->device);
   const long long nl = s->light_end - s->light_begin;
   if (nl == 0) return 0;
-  const long long chunk = chunk_rays_for(s->exact, s->shape, out);
+  long long rays = 0;
+  for (int i = 0; i < n; ++i) rays += (long long)s->templates[ids[i]].num_facets * nl;
+  const int chunk_iters = chunk_iters_for(s->exact, s->shape, out, rays);
+  const long long chunk = 32LL * chunk_iters;
   auto chunks_of = [&](int id) { return ((long long)s->templates[id].num_facets * nl + chunk - 1) / chunk; };
   bool same = s->cache_valid && s->cached_lights == nl && s->cached_chunk == chunk && (int)s->cached_ids.size() == n &&
               std::equal(ids, ids + n, s->cached_ids.begin());
@@ -539,11 +554,11 @@ long long trace_ids(qmcrt_scene* s, const int* ids, int n, cudaStream_t stream, 
     if (s->d_work.bytes < sizeof(unsigned long long)) s->d_work.alloc(sizeof(unsigned long long));
     work = s->d_work.as<unsigned long long>();
   }
-  cuda_check(run_trace(s, p, out, stream, work), "trace kernel");
+  cuda_check(launch_trace_mode(s->exact, p, out, stream, s->shape, chunk_iters, work), "trace kernel");
   return total;
 }
 
-int trace_chunk_rays() { return qm::trace_chunk_rays_fast(); }
+int trace_chunk_rays() { return qm::kChunk; }
 
 }  // namespace qrt
 
@@ -1201,7 +1216,7 @@ int qmcrt_debug_hit_records(qmcrt_scene* s, int id, int fb, int fe, int lb, int 
     p.record_task = 0;
     p.record_facet_begin = fb;
     p.record_facet_end = fe;
-    cuda_check(run_trace(s, p, 1, 0), "record kernel");
+    cuda_check(launch_trace_mode(s->exact, p, 1, 0, 0, qm::kChunkIters), "record kernel");
     cuda_check(cudaMemcpy(codes, rec.p, count * sizeof(int32_t), cudaMemcpyDeviceToHost), "readback");
   });
 }

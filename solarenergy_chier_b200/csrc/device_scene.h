@@ -102,6 +102,10 @@ enum DiagSlot { kDiagClamped = 0, kDiagDdaCap = 1, kDiagSlots = 4 };
 #endif
 constexpr int kChunkIters = QM_CHUNK_ITERS;
 constexpr int kChunk = 32 * kChunkIters;
+// Chunks of flux launches too small to fill the GPU with the larger one
+// (qrt::chunk_iters_for): a chunk's iterations run one after another.
+constexpr int kSmallChunkIters = 8;
+constexpr int kMediumChunkIters = 16;
 
 struct TraceParams {
   const DevGrid* grids;

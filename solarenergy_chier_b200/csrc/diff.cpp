@@ -114,6 +114,7 @@ void diff_create(qmcrt_scene* s, const float* sun_dirs, int n_suns, float sigma_
   if (qmcrt_batch_create(scenes.data(), 1, scene_of.data(), sun_dirs, n_suns, &d->batch) != QMCRT_OK)
     throw ApiError(QMCRT_ERR_INVALID, qmcrt_last_error());
   qmcrt_batch* b = d->batch;
+  b->hit_record_chunks = true;
   DeviceGuard guard(b->device);
   for (const auto& I : b->inst) {
     for (int h = 0; h < d->H; ++h) {

@@ -467,7 +467,8 @@ __device__ __forceinline__ void splat_bilinear(const DevReceiver& R, float X, fl
 #define QM_TRACE_ARGS TraceParams p
 #endif
 
-template <int kOut>
+// kIters: warp-chunk iterations (kChunkIters, fewer in small flux launches).
+template <int kOut, int kIters = kChunkIters>
 #ifndef QM_TRACE_MIN_BLOCKS
 #define QM_TRACE_MIN_BLOCKS 4
 #endif
@@ -501,15 +502,15 @@ __global__ void __launch_bounds__(kThreads, QM_TRACE_MIN_BLOCKS) trace_kernel(QM
   int t, r0, r_end;
   if (kOut == kOutRecord) {
     const long long span = (long long)(p.record_facet_end - p.record_facet_begin) * nl;
-    if (warp * kChunk >= span) return;
+    if (warp * (32 * kIters) >= span) return;
     t = p.record_task;
-    r0 = p.record_facet_begin * nl + (int)warp * kChunk;
+    r0 = p.record_facet_begin * nl + (int)warp * (32 * kIters);
     r_end = p.record_facet_end * nl;
   } else {
     const long long chunk = p.chunk_begin + warp;
     if (chunk >= p.total_facets) return;  // total_facets holds the end chunk
     t = find_task(p.facet_prefix, p.num_tasks, chunk);
-    r0 = (int)(chunk - __ldg(p.facet_prefix + t)) * kChunk;
+    r0 = (int)(chunk - __ldg(p.facet_prefix + t)) * (32 * kIters);
     r_end = p.tasks[t].num_facets * nl;
   }
   // The task stays in global memory (L1-resident) and is read where used.
@@ -526,7 +527,7 @@ __global__ void __launch_bounds__(kThreads, QM_TRACE_MIN_BLOCKS) trace_kernel(QM
   int f = (r0 + lane) / nl;
   int l = (r0 + lane) - f * nl;
   const int q32 = p.lights_q32, r32 = p.lights_r32;
-  const int iters = min(kChunkIters, (r_end - r0 + 31) >> 5);  // warp-uniform
+  const int iters = min(kIters, (r_end - r0 + 31) >> 5);  // warp-uniform
 
   unsigned flags = 0;
   double power = 0.0;
@@ -653,7 +654,7 @@ __global__ void __launch_bounds__(kThreads, QM_TRACE_MIN_BLOCKS) trace_kernel(QM
     }
     if (kOut == kOutSplat || kOut == kOutBits) {
       const unsigned bits = __ballot_sync(0xffffffffu, hit);
-      if (lane == 0 && p.hit_bits) p.hit_bits[warp * kChunkIters + it] = bits;
+      if (lane == 0 && p.hit_bits) p.hit_bits[warp * kIters + it] = bits;
     }
     f += q32;
     l += r32;
@@ -697,10 +698,8 @@ cudaError_t QM_SYM(launch_facets)(const DevTask& task, float3* origins, float3* 
   return cudaGetLastError();
 }
 
-int QM_SYM(trace_chunk_rays)() { return kChunk; }
-
 cudaError_t QM_SYM(launch_trace)(const TraceParams& params, int out, cudaStream_t stream,
-                                 unsigned long long* work_counter) {
+                                 unsigned long long* work_counter, int chunk_iters) {
   const int threads = kThreads;
   const long long nl = params.light_end - params.light_begin;
   if (nl <= 0) return cudaSuccess;
@@ -740,7 +739,20 @@ cudaError_t QM_SYM(launch_trace)(const TraceParams& params, int out, cudaStream_
     case kOutRecord: trace_kernel<kOutRecord><<<(unsigned)blocks, threads, 0, stream>>>(QM_TRACE_LAUNCH_ARGS); break;
     case kOutSplat: trace_kernel<kOutSplat><<<(unsigned)blocks, threads, 0, stream>>>(QM_TRACE_LAUNCH_ARGS); break;
     case kOutBits: trace_kernel<kOutBits><<<(unsigned)blocks, threads, 0, stream>>>(QM_TRACE_LAUNCH_ARGS); break;
-    default: trace_kernel<kOutFlux><<<(unsigned)blocks, threads, 0, stream>>>(QM_TRACE_LAUNCH_ARGS); break;
+    default:
+#if QM_CHUNK_ITERS == 64 && QM_TRACE_THREADS != 64 && !defined(QM_TRACE_PERSISTENT)
+      if (chunk_iters == kSmallChunkIters) {
+        trace_kernel<kOutFlux, kSmallChunkIters><<<(unsigned)blocks, threads, 0, stream>>>(QM_TRACE_LAUNCH_ARGS);
+        break;
+      }
+      if (chunk_iters == kMediumChunkIters) {
+        trace_kernel<kOutFlux, kMediumChunkIters><<<(unsigned)blocks, threads, 0, stream>>>(QM_TRACE_LAUNCH_ARGS);
+        break;
+      }
+#endif
+      if (chunk_iters != kChunkIters) return cudaErrorInvalidValue;
+      trace_kernel<kOutFlux><<<(unsigned)blocks, threads, 0, stream>>>(QM_TRACE_LAUNCH_ARGS);
+      break;
   }
   return cudaGetLastError();
 }

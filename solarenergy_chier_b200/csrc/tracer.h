@@ -16,44 +16,36 @@ namespace qm {
 // ignore it.  It is a kernel argument of that build alone, not a TraceParams
 // field: growing the kernels' parameter block changed the register
 // allocation of every build and cost 2.5-3.7 % of their throughput.
+// chunk_iters: warp-chunk iterations of a flux launch, the build's own or (one
+// launch per chunk, 64-iteration builds) kSmallChunkIters or kMediumChunkIters.
 cudaError_t launch_trace_fast(const TraceParams& p, int out, cudaStream_t stream,
-                              unsigned long long* work_counter = nullptr);
+                              unsigned long long* work_counter, int chunk_iters);
 cudaError_t launch_trace_exact(const TraceParams& p, int out, cudaStream_t stream,
-                              unsigned long long* work_counter = nullptr);
+                              unsigned long long* work_counter, int chunk_iters);
 // Production build limited to 64 registers (four 256-thread blocks per SM).
 cudaError_t launch_trace_fast4(const TraceParams& p, int out, cudaStream_t stream,
-                              unsigned long long* work_counter = nullptr);
+                              unsigned long long* work_counter, int chunk_iters);
 // Production build in other launch shapes (the autotuner's candidates):
 // 32-iteration and 128-iteration warp chunks, two-warp blocks.
 cudaError_t launch_trace_fast_c32(const TraceParams& p, int out, cudaStream_t stream,
-                              unsigned long long* work_counter = nullptr);
+                              unsigned long long* work_counter, int chunk_iters);
 cudaError_t launch_trace_fast_c128(const TraceParams& p, int out, cudaStream_t stream,
-                              unsigned long long* work_counter = nullptr);
+                              unsigned long long* work_counter, int chunk_iters);
 cudaError_t launch_trace_fast_t64(const TraceParams& p, int out, cudaStream_t stream,
-                              unsigned long long* work_counter = nullptr);
-int trace_chunk_rays_fast_c32();
-int trace_chunk_rays_fast_c128();
-int trace_chunk_rays_fast_t64();
+                              unsigned long long* work_counter, int chunk_iters);
 // Persistent launch shape: resident one-warp blocks taking warp chunks from a
 // work counter in flux launches (without one it launches one warp per chunk).
 cudaError_t launch_trace_fast_ps(const TraceParams& p, int out, cudaStream_t stream,
-                              unsigned long long* work_counter = nullptr);
-int trace_chunk_rays_fast_ps();
+                              unsigned long long* work_counter, int chunk_iters);
 // Production build with the arithmetic after the receiver's decisions
 // approximated (hit point, pixel position, energy).
 cudaError_t launch_trace_rx(const TraceParams& p, int out, cudaStream_t stream,
-                              unsigned long long* work_counter = nullptr);
-int trace_chunk_rays_rx();
+                              unsigned long long* work_counter, int chunk_iters);
 // Production build with approximate per-ray arithmetic after the shadow test
 // (FMA contraction, hardware reciprocal square root, approximate divisions).
 cudaError_t launch_trace_approx(const TraceParams& p, int out, cudaStream_t stream,
-                              unsigned long long* work_counter = nullptr);
-int trace_chunk_rays_approx();
+                              unsigned long long* work_counter, int chunk_iters);
 cudaError_t launch_facets_approx(const DevTask& task, float3* origins, float3* normals, cudaStream_t stream);
-// Rays per warp chunk; TraceParams::facet_prefix counts chunks per task.
-int trace_chunk_rays_fast();
-int trace_chunk_rays_exact();
-int trace_chunk_rays_fast4();
 
 // Micro-facet centres and normals of one heliostat, from the same device
 // function the tracer evaluates per facet.

@@ -132,6 +132,28 @@ def test_uneven_fields_batch_equals_plain(tmp_path):
         assert np.allclose(gper, per, rtol=1e-9, atol=0)
 
 
+@pytest.mark.parametrize("heliostats,lights", [(1, 1), (1, 37), (3, 33), (1, 994), (1, 995), (50, 199), (50, 200)])
+def test_chunk_sizes_of_small_launches(heliostats, lights, tmp_path):
+    """Flux launches below 6.4 M and 64 M rays take 8- and 16-iteration warp
+    chunks; either side of both limits (and chunks that end inside a facet)
+    they give what 64-iteration chunks of another launch shape do: the same
+    flux up to float atomic order (L1 <= 1e-6) and FP64 powers (1e-12)."""
+    f = synth.small_field(tmp_path, seed=1)
+    s = q.Scene(f.scene, f.config, device=0, seed=2)
+    s.set_light_range(5, 5 + lights)
+    ids = list(range(heliostats))
+    out = []
+    for shape in (3, 0):  # two-warp blocks of 64-iteration chunks, then the default shape
+        s.set_launch_shape(shape)
+        s.clear()
+        s.clear_power()
+        s.trace(ids)
+        out.append((s.image(0).astype(np.float64), s.power()[0]))
+    (img0, p0), (img, p) = out
+    assert p0.sum() > 0 and np.abs(img - img0).sum() <= 1e-6 * img0.sum()
+    np.testing.assert_allclose(p, p0, rtol=1e-12, atol=0)
+
+
 def test_every_launch_shape_gives_the_same_result(fields, tmp_path):
     """The autotuner's candidates (launch shapes of the production build:
     block widths, warp chunks of 32, 64 or 128 iterations) change only how
