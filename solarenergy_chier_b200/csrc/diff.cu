@@ -12,11 +12,13 @@
 // dL/dD = P), a ray depositing energy e at pixel position (X, Y) contributes
 //   dL/dtheta = e (dPb/dX dX/dtheta + dPb/dY dY/dtheta) + Pb de/dtheta,
 // Pb the bilinear interpolation of P at (X, Y) -- the exact derivative of
-// the discretised forward.  (X, Y) and e are differentiated forward-mode
-// (value + 4 tangents) from the heliostat's parameters through its normal
-// and frame, the facet position and normal, the slope-error normal, the
-// reflection, the receiver intersection (implicitly: the hit point stays on
-// the receiver surface) and the energy (cosine and atmospheric attenuation).
+// the discretised forward.  The chain from the heliostat's normal and frame
+// over the facet position and normal, the slope-error normal, the reflection,
+// the receiver intersection (implicitly: the hit point stays on the receiver
+// surface) and the energy (cosine and atmospheric attenuation) is run
+// backwards per ray, down to the heliostat's frame axes, whose derivatives
+// with respect to its four parameters (forward-mode, once per heliostat) are
+// applied to a warp chunk's sums.
 // Shadowing and blocking are treated as constants (indicators detached):
 // only rays whose hit bit the forward set contribute, and no grid walk is
 // repeated.  The receiver's own edges (a cylinder's silhouette, the image's
@@ -41,93 +43,133 @@ constexpr float kEdgeBand = 1.0f;
 constexpr float kTwoPi = 6.28318530717959f;
 
 // ---- value + tangent arithmetic ----------------------------------------------
-__device__ __forceinline__ Dual dc(float v) {
-  Dual r;
+template <int N>
+__device__ __forceinline__ DualT<N> dc(float v) {
+  DualT<N> r;
   r.v = v;
 #pragma unroll
-  for (int k = 0; k < K; ++k) r.d[k] = 0.0f;
+  for (int k = 0; k < N; ++k) r.d[k] = 0.0f;
   return r;
 }
-__device__ __forceinline__ Dual dvar(float v, int k) {
-  Dual r = dc(v);
+template <int N>
+__device__ __forceinline__ DualT<N> dvar(float v, int k) {
+  DualT<N> r = dc<N>(v);
   r.d[k] = 1.0f;
   return r;
 }
-__device__ __forceinline__ Dual operator+(Dual a, Dual b) {
-  Dual r;
+template <int N>
+__device__ __forceinline__ DualT<N> operator+(DualT<N> a, DualT<N> b) {
+  DualT<N> r;
   r.v = a.v + b.v;
 #pragma unroll
-  for (int k = 0; k < K; ++k) r.d[k] = a.d[k] + b.d[k];
+  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] + b.d[k];
   return r;
 }
-__device__ __forceinline__ Dual operator-(Dual a, Dual b) {
-  Dual r;
+template <int N>
+__device__ __forceinline__ DualT<N> operator-(DualT<N> a, DualT<N> b) {
+  DualT<N> r;
   r.v = a.v - b.v;
 #pragma unroll
-  for (int k = 0; k < K; ++k) r.d[k] = a.d[k] - b.d[k];
+  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] - b.d[k];
   return r;
 }
-__device__ __forceinline__ Dual operator-(Dual a) {
-  Dual r;
+template <int N>
+__device__ __forceinline__ DualT<N> operator-(DualT<N> a) {
+  DualT<N> r;
   r.v = -a.v;
 #pragma unroll
-  for (int k = 0; k < K; ++k) r.d[k] = -a.d[k];
+  for (int k = 0; k < N; ++k) r.d[k] = -a.d[k];
   return r;
 }
-__device__ __forceinline__ Dual operator*(Dual a, Dual b) {
-  Dual r;
+template <int N>
+__device__ __forceinline__ DualT<N> operator*(DualT<N> a, DualT<N> b) {
+  DualT<N> r;
   r.v = a.v * b.v;
 #pragma unroll
-  for (int k = 0; k < K; ++k) r.d[k] = a.d[k] * b.v + a.v * b.d[k];
+  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] * b.v + a.v * b.d[k];
   return r;
 }
-__device__ __forceinline__ Dual operator*(Dual a, float s) {
-  Dual r;
+template <int N>
+__device__ __forceinline__ DualT<N> operator*(DualT<N> a, float s) {
+  DualT<N> r;
   r.v = a.v * s;
 #pragma unroll
-  for (int k = 0; k < K; ++k) r.d[k] = a.d[k] * s;
+  for (int k = 0; k < N; ++k) r.d[k] = a.d[k] * s;
   return r;
 }
 // 1 / sqrt(a)
-__device__ __forceinline__ Dual drsqrt(Dual a) {
+template <int N>
+__device__ __forceinline__ DualT<N> drsqrt(DualT<N> a) {
   const float r = rsqrtf(a.v);
-  const float dr = -0.5f * r * r * r;
-  Dual o;
+  DualT<N> o;
   o.v = r;
+  if constexpr (N > 0) {
+    const float dr = -0.5f * r * r * r;
 #pragma unroll
-  for (int k = 0; k < K; ++k) o.d[k] = dr * a.d[k];
+    for (int k = 0; k < N; ++k) o.d[k] = dr * a.d[k];
+  }
   return o;
 }
 
-__device__ __forceinline__ Dual3 d3(float3 c) { return Dual3{dc(c.x), dc(c.y), dc(c.z)}; }
-__device__ __forceinline__ float3 val(const Dual3& a) { return make_float3(a.x.v, a.y.v, a.z.v); }
-__device__ __forceinline__ Dual3 operator+(const Dual3& a, const Dual3& b) { return Dual3{a.x + b.x, a.y + b.y, a.z + b.z}; }
-__device__ __forceinline__ Dual3 operator-(const Dual3& a, const Dual3& b) { return Dual3{a.x - b.x, a.y - b.y, a.z - b.z}; }
-__device__ __forceinline__ Dual3 operator-(const Dual3& a) { return Dual3{-a.x, -a.y, -a.z}; }
-__device__ __forceinline__ Dual3 operator*(const Dual3& a, Dual s) { return Dual3{a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ Dual3 operator*(const Dual3& a, float s) { return Dual3{a.x * s, a.y * s, a.z * s}; }
-__device__ __forceinline__ Dual dot(const Dual3& a, const Dual3& b) { return a.x * b.x + a.y * b.y + a.z * b.z; }
-__device__ __forceinline__ Dual3 cross(const Dual3& a, const Dual3& b) {
-  return Dual3{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+template <int N>
+__device__ __forceinline__ Dual3T<N> d3(float3 c) {
+  return Dual3T<N>{dc<N>(c.x), dc<N>(c.y), dc<N>(c.z)};
 }
-__device__ __forceinline__ Dual3 normalize(const Dual3& a) { return a * drsqrt(dot(a, a)); }
+template <int N>
+__device__ __forceinline__ float3 val(const Dual3T<N>& a) {
+  return make_float3(a.x.v, a.y.v, a.z.v);
+}
+template <int N>
+__device__ __forceinline__ Dual3T<N> operator+(const Dual3T<N>& a, const Dual3T<N>& b) {
+  return Dual3T<N>{a.x + b.x, a.y + b.y, a.z + b.z};
+}
+template <int N>
+__device__ __forceinline__ Dual3T<N> operator-(const Dual3T<N>& a, const Dual3T<N>& b) {
+  return Dual3T<N>{a.x - b.x, a.y - b.y, a.z - b.z};
+}
+template <int N>
+__device__ __forceinline__ Dual3T<N> operator-(const Dual3T<N>& a) {
+  return Dual3T<N>{-a.x, -a.y, -a.z};
+}
+template <int N>
+__device__ __forceinline__ Dual3T<N> operator*(const Dual3T<N>& a, DualT<N> s) {
+  return Dual3T<N>{a.x * s, a.y * s, a.z * s};
+}
+template <int N>
+__device__ __forceinline__ Dual3T<N> operator*(const Dual3T<N>& a, float s) {
+  return Dual3T<N>{a.x * s, a.y * s, a.z * s};
+}
+template <int N>
+__device__ __forceinline__ DualT<N> dot(const Dual3T<N>& a, const Dual3T<N>& b) {
+  return a.x * b.x + a.y * b.y + a.z * b.z;
+}
+template <int N>
+__device__ __forceinline__ Dual3T<N> cross(const Dual3T<N>& a, const Dual3T<N>& b) {
+  return Dual3T<N>{a.y * b.z - a.z * b.y, a.z * b.x - a.x * b.z, a.x * b.y - a.y * b.x};
+}
+template <int N>
+__device__ __forceinline__ Dual3T<N> normalize(const Dual3T<N>& a) {
+  return a * drsqrt(dot(a, a));
+}
 
 // Frame (u, n, v) of a normal, as qm::make_frame (Util/global_function.cuh:19-36
 // and the flipped focus-flat variant), with tangents.
-struct DFrame {
-  Dual3 u, n, v;
+template <int N>
+struct DFrameT {
+  Dual3T<N> u, n, v;
   bool identity;
 };
-__device__ __forceinline__ DFrame make_dframe(const Dual3& n, bool flip) {
-  DFrame f;
+template <int N>
+__device__ __forceinline__ DFrameT<N> make_dframe(const Dual3T<N>& n, bool flip) {
+  DFrameT<N> f;
   f.n = n;
   f.identity = qm_below_eps(fabsf(n.x.v)) && qm_below_eps(fabsf(n.z.v));
   if (f.identity) {
-    f.u = d3(make_float3(1.f, 0.f, 0.f));
-    f.v = d3(make_float3(0.f, 0.f, 1.f));
+    f.u = d3<N>(make_float3(1.f, 0.f, 0.f));
+    f.v = d3<N>(make_float3(0.f, 0.f, 1.f));
     return f;
   }
-  f.u = normalize(cross(d3(make_float3(0.f, 1.f, 0.f)), n));
+  f.u = normalize(cross(d3<N>(make_float3(0.f, 1.f, 0.f)), n));
   f.v = normalize(cross(f.u, n));
   if (flip && n.z.v < 0) {
     f.u = -f.u;
@@ -135,8 +177,9 @@ __device__ __forceinline__ DFrame make_dframe(const Dual3& n, bool flip) {
   }
   return f;
 }
-__device__ __forceinline__ Dual3 to_world(const DFrame& f, float3 d) {
-  if (f.identity) return d3(d);
+template <int N>
+__device__ __forceinline__ Dual3T<N> to_world(const DFrameT<N>& f, float3 d) {
+  if (f.identity) return d3<N>(d);
   return f.u * d.x + f.n * d.y + f.v * d.z;
 }
 
@@ -147,7 +190,7 @@ __global__ void diff_prep_kernel(const PrepItem* items, int n, const DevTask* ta
   const PrepItem it = items[i];
   const DevTask& T = tasks[it.task];
   // aim point a = focus + du aim_u + dv aim_v
-  Dual3 a = d3(make_float3(it.focus.x + it.aim_u.x * it.aim_offset.x + it.aim_v.x * it.aim_offset.y,
+  Dual3T<K> a = d3<K>(make_float3(it.focus.x + it.aim_u.x * it.aim_offset.x + it.aim_v.x * it.aim_offset.y,
                            it.focus.y + it.aim_u.y * it.aim_offset.x + it.aim_v.y * it.aim_offset.y,
                            it.focus.z + it.aim_u.z * it.aim_offset.x + it.aim_v.z * it.aim_offset.y));
   a.x.d[0] = it.aim_u.x;
@@ -156,11 +199,12 @@ __global__ void diff_prep_kernel(const PrepItem* items, int n, const DevTask* ta
   a.x.d[1] = it.aim_v.x;
   a.y.d[1] = it.aim_v.y;
   a.z.d[1] = it.aim_v.z;
-  const Dual3 r = normalize(a - d3(T.pos));
-  const Dual3 n0 = normalize(r - d3(it.sun_dir));
-  const DFrame f0 = make_dframe(n0, false);
-  const Dual3 nrm = normalize(n0 + f0.u * dvar(it.normal_offset.x, 2) + f0.v * dvar(it.normal_offset.y, 3));
-  const DFrame hf = make_dframe(nrm, T.type == 1);
+  const Dual3T<K> r = normalize(a - d3<K>(T.pos));
+  const Dual3T<K> n0 = normalize(r - d3<K>(it.sun_dir));
+  const DFrameT<K> f0 = make_dframe(n0, false);
+  const Dual3T<K> nrm =
+      normalize(n0 + f0.u * dvar<K>(it.normal_offset.x, 2) + f0.v * dvar<K>(it.normal_offset.y, 3));
+  const DFrameT<K> hf = make_dframe(nrm, T.type == 1);
   DiffTask o;
   o.n = nrm;
   o.u = hf.u;
@@ -171,71 +215,122 @@ __global__ void diff_prep_kernel(const PrepItem* items, int n, const DevTask* ta
 }
 
 // ---- adjoint ------------------------------------------------------------------
-__device__ __forceinline__ float sample_p(const DevReceiver& R, int c, int r) {
+// P at the four pixels around pixel position (xs + 0.5, ys + 0.5), with the
+// forward deposit's wrap / zero conventions.
+struct Quad {
+  float p00, p10, p01, p11;  // p<column><row>
+  float fx, fy;
+};
+__device__ __forceinline__ Quad sample_quad(const DevReceiver& R, float xs, float ys) {
+  const float x0 = floorf(xs), y0 = floorf(ys);
+  Quad q;
+  q.fx = xs - x0;
+  q.fy = ys - y0;
   const int w = R.resolution.x, h = R.resolution.y;
-  if (R.type == 1) c = c < 0 ? c + w : (c >= w ? c - w : c);
-  if (c < 0 || c >= w || r < 0 || r >= h) return 0.0f;
-  return __ldg(R.image + r * w + c);
+  int c0 = (int)x0, c1 = c0 + 1;
+  const int r0 = (int)y0, r1 = r0 + 1;
+  if (R.type == 1) {
+    c0 = c0 < 0 ? c0 + w : (c0 >= w ? c0 - w : c0);
+    c1 = c1 < 0 ? c1 + w : (c1 >= w ? c1 - w : c1);
+  }
+  const bool in0 = (unsigned)c0 < (unsigned)w, in1 = (unsigned)c1 < (unsigned)w;
+  const bool up = (unsigned)r0 < (unsigned)h, down = (unsigned)r1 < (unsigned)h;
+  const float* row = R.image + (long long)r0 * w;
+  q.p00 = up && in0 ? __ldg(row + c0) : 0.0f;
+  q.p10 = up && in1 ? __ldg(row + c1) : 0.0f;
+  q.p01 = down && in0 ? __ldg(row + w + c0) : 0.0f;
+  q.p11 = down && in1 ? __ldg(row + w + c1) : 0.0f;
+  return q;
+}
+__device__ __forceinline__ float bilinear(const Quad& q) {
+  return (1 - q.fx) * (1 - q.fy) * q.p00 + q.fx * (1 - q.fy) * q.p10 + (1 - q.fx) * q.fy * q.p01 + q.fx * q.fy * q.p11;
 }
 
-// Bilinear interpolation of P at continuous pixel position (X, Y), with the
-// forward deposit's wrap / zero conventions.
-__device__ __forceinline__ float bilinear_p(const DevReceiver& R, float X, float Y) {
-  const float xs = X - 0.5f, ys = Y - 0.5f;
-  const float x0 = floorf(xs), y0 = floorf(ys);
-  const float fx = xs - x0, fy = ys - y0;
-  const int c0 = (int)x0, r0 = (int)y0;
-  return (1 - fx) * (1 - fy) * sample_p(R, c0, r0) + fx * (1 - fy) * sample_p(R, c0 + 1, r0) +
-         (1 - fx) * fy * sample_p(R, c0, r0 + 1) + fx * fy * sample_p(R, c0 + 1, r0 + 1);
+// Bilinear interpolation of P at continuous pixel position (X, Y).
+__device__ __noinline__ float bilinear_p(const DevReceiver& R, float X, float Y) {
+  return bilinear(sample_quad(R, X - 0.5f, Y - 0.5f));
 }
 
 // What the rays of one facet share: its origin and the frame of its normal
-// (the slope-error perturbation's frame), as functions of the heliostat's
-// parameters, and its two pool offsets.
-struct FacetDual {
-  Dual3 origin;
-  DFrame pframe;
+// (the slope-error perturbation's frame), its point and its sub-heliostat's
+// normal in the heliostat's local frame, and its two pool offsets.
+struct Facet {
+  float3 origin, u, n, v, local, local_normal;
+  bool identity;
   int g0, g1;
 };
 
-__device__ __forceinline__ FacetDual facet_dual(const DevTask& T, const DiffTask& DT, int f) {
-  float3 local, ln;
-  const bool focus_flat = facet_local(T, f, local, ln);
-  DFrame hf;
-  hf.u = DT.u;
-  hf.n = DT.fn;
-  hf.v = DT.v;
+// The values follow the dual arithmetic of the preparation (value parts).
+__device__ __forceinline__ Facet make_facet(const DevTask& T, const DiffTask& DT, int f) {
+  Facet fd;
+  const bool focus_flat = facet_local(T, f, fd.local, fd.local_normal);
+  DFrameT<0> hf;
+  hf.u = d3<0>(val(DT.u));
+  hf.n = d3<0>(val(DT.fn));
+  hf.v = d3<0>(val(DT.v));
   hf.identity = DT.identity != 0;
-  FacetDual fd;
-  fd.origin = to_world(hf, local) + d3(T.pos);
-  const Dual3 fnormal = focus_flat ? to_world(hf, ln) : DT.n;
-  fd.pframe = make_dframe(fnormal, false);
+  fd.origin = val(to_world(hf, fd.local) + d3<0>(T.pos));
+  const Dual3T<0> normal = focus_flat ? to_world(hf, fd.local_normal) : d3<0>(val(DT.n));
+  const DFrameT<0> fr = make_dframe(normal, false);
+  fd.u = val(fr.u);
+  fd.n = val(fr.n);
+  fd.v = val(fr.v);
+  fd.identity = fr.identity;
   fd.g0 = __ldg(T.offsets + f);
   fd.g1 = __ldg(T.offsets + (f + 1) % T.pool_size);
   return fd;
 }
 
-// Contribution of one ray (facet fd, light lab) that hit the receiver in the
-// forward.
-__device__ __forceinline__ void ray_adjoint(const DevTask& T, const DevReceiver& R, const FacetDual& fd, int lab,
-                                            float g[K]) {
-  const Dual3& origin = fd.origin;
+// Adjoint of the heliostat's facet frame, one lane's sum: row j is d/d(axis j).
+struct FrameSum {
+  float3 u, n, v;
+};
+__device__ __forceinline__ void add_outer(FrameSum& s, float3 a, float3 l) {
+  s.u.x += a.x * l.x; s.u.y += a.y * l.x; s.u.z += a.z * l.x;
+  s.n.x += a.x * l.y; s.n.y += a.y * l.y; s.n.z += a.z * l.y;
+  s.v.x += a.x * l.z; s.v.y += a.y * l.z; s.v.z += a.z * l.z;
+}
+__device__ __forceinline__ float3 axpy(float s, float3 x, float3 y) {
+  return make_float3(s * x.x + y.x, s * x.y + y.y, s * x.z + y.z);
+}
+
+// What a chunk's rays share, in shared memory: read per ray, and a read from
+// the task and receiver tables would wait on the L1.
+struct ChunkConstants {
+  DevReceiver R;
+  const float4* samples;
+  const float4* perturbations;
+  float factor;
+};
+
+// Adds the contribution of one ray (facet fd, light lab) that hit the
+// receiver in the forward to `sum`.
+__device__ __forceinline__ void ray_adjoint(const ChunkConstants& T, const Facet& fd, int lab, FrameSum& sum) {
+  const DevReceiver& R = T.R;
+  const float3 o = fd.origin;
   const float3 din = xyz(__ldg(T.samples + fd.g0 + lab));
   const float3 pert = xyz(__ldg(T.perturbations + fd.g1 + lab));
-  const Dual3 np = normalize(to_world(fd.pframe, pert));
-  const Dual3 in = d3(make_float3(-din.x, -din.y, -din.z));
-  const Dual3 rd = normalize(in - np * (dot(np, in) * 2.0f));
-  const float3 o = val(origin), d = val(rd);
+  DFrameT<0> fr;
+  fr.u = d3<0>(fd.u);
+  fr.n = d3<0>(fd.n);
+  fr.v = d3<0>(fd.v);
+  fr.identity = fd.identity;
+  const Dual3T<0> slope = to_world(fr, pert);
+  const Dual3T<0> dnp = normalize(slope);
+  const Dual3T<0> din3 = d3<0>(make_float3(-din.x, -din.y, -din.z));
+  const DualT<0> c0 = dot(dnp, din3);
+  const Dual3T<0> drd = normalize(din3 - dnp * (c0 * 2.0f));
+  const float3 d = val(drd), np = val(dnp), in = val(din3);
   float t, u, v;
   // The receiver test with its decisions rounded as the forward's and the
   // hit point, (u, v) and distance in approximate arithmetic: the direction
-  // here is the dual chain's contracted value, not the forward's, so the
-  // exact position arithmetic would buy nothing.  A ray the rounding moves
-  // off the receiver edge adds nothing.
+  // here is a contracted value, not the forward's, so the exact position
+  // arithmetic would buy nothing.  A ray the rounding moves off the receiver
+  // edge adds nothing.
   if (!receiver_hit_rx(R, o, d, t, u, v)) return;
   // energy |rd . np| eta(t) factor (receiverIntersectionUtil.cuh:17-34)
-  const Dual c = dot(rd, np);
-  const float sgn = c.v >= 0.0f ? 1.0f : -1.0f;
+  const float c = dot(drd, dnp).v;
+  const float sgn = c >= 0.0f ? 1.0f : -1.0f;
   float eta, deta;
   if (t <= 1000.0f) {
     eta = 0.99331f - 0.0001176f * t + 1.97e-8f * t * t;
@@ -244,121 +339,124 @@ __device__ __forceinline__ void ray_adjoint(const DevTask& T, const DevReceiver&
     eta = expf(-0.0001106f * t);
     deta = -0.0001106f * eta;
   }
-  const float e = fabsf(c.v) * eta * T.factor;
-  // bilinear P at the deposit position (as the forward's splat)
-  const float X = v * (float)R.resolution.x, Y = u * (float)R.resolution.y;
-  const float xs = X - 0.5f, ys = Y - 0.5f;
-  const float x0 = floorf(xs), y0 = floorf(ys);
-  const float fx = xs - x0, fy = ys - y0;
-  const int c0 = (int)x0, r0 = (int)y0;
-  const float p00 = sample_p(R, c0, r0), p10 = sample_p(R, c0 + 1, r0);
-  const float p01 = sample_p(R, c0, r0 + 1), p11 = sample_p(R, c0 + 1, r0 + 1);
-  const float pb = (1 - fx) * (1 - fy) * p00 + fx * (1 - fy) * p10 + (1 - fx) * fy * p01 + fx * fy * p11;
-  const float dpx = (1 - fy) * (p10 - p00) + fy * (p11 - p01);
-  const float dpy = (1 - fx) * (p01 - p00) + fx * (p11 - p10);
-
-  float dX[K], dY[K], dt[K];
+  const float e = fabsf(c) * eta * T.factor;
+  // The adjoints of the hit point's path: of the origin, of the reflected
+  // direction and of c = rd . np.
+  float3 obar, rdbar;
+  float cbar = 0.0f;
+  bool band = false;
+  float x = 0.0f, z = 0.0f, den = 0.0f, rr = 0.0f, dxz2 = 0.0f;
   if (R.type == 1) {
     const float3 p = make_float3(o.x + t * d.x, o.y + t * d.y, o.z + t * d.z);
-    const float x = p.x - R.pos.x, z = p.z - R.pos.z;
-    const float den = x * d.x + z * d.z;
-    const float rr = x * x + z * z;
-    const float dxz2 = d.x * d.x + d.z * d.z;
+    x = p.x - R.pos.x;
+    z = p.z - R.pos.z;
+    den = x * d.x + z * d.z;
+    rr = x * x + z * z;
+    dxz2 = d.x * d.x + d.z * d.z;
     if (!(rr > 0.0f) || !(dxz2 > 0.0f)) return;
-    if (!(fabsf(den) > kGrazing * sqrtf(rr * dxz2))) {
-      // Silhouette band: rays whose impact parameter b (distance of the
-      // ray's horizontal line from the axis) lies within w of the radius
-      // (|cos incidence| < kGrazing).  Their interior derivative grows as
-      // 1/cos(incidence) and is not summed; across the band it integrates
-      // to rho e v (P(silhouette) - P(inner band edge)), and the boundary
-      // term of rays crossing the silhouette is -rho e v P(silhouette), so
-      // together the band contributes -rho e v P(inner band edge), with
-      // v = d|b|/dtheta and rho ~ (rays in the band) / w.  P is taken where
-      // this ray's line would meet the cylinder with impact parameter R - w.
-      const float radius = R.size.x;
-      const float w = radius * (1.0f - sqrtf(1.0f - kGrazing * kGrazing));
-      const Dual ox = origin.x - dc(R.pos.x), oz = origin.z - dc(R.pos.z);
-      const Dual b = (ox * rd.z - oz * rd.x) * drsqrt(rd.x * rd.x + rd.z * rd.z);
-      const float out = b.v >= 0.0f ? 1.0f : -1.0f;
-      const float inv_dxz = rsqrtf(dxz2);
-      const float hx = d.x * inv_dxz, hz = d.z * inv_dxz;  // horizontal unit direction
-      const float tca = -((o.x - R.pos.x) * d.x + (o.z - R.pos.z) * d.z) / dxz2;
-      const float cx = o.x + tca * d.x - R.pos.x, cz = o.z + tca * d.z - R.pos.z;  // closest approach
-      const float cl = sqrtf(cx * cx + cz * cz);
-      const float ux = cl > 0.0f ? cx / cl : -hz, uz = cl > 0.0f ? cz / cl : hx;
-      const float back = radius * kGrazing;  // sqrt(R^2 - (R - w)^2)
-      const float ex = (radius - w) * ux - back * hx, ez = (radius - w) * uz - back * hz;
-      float phi = atan2f(ez, ex);
-      if (phi < 0.0f) phi += kTwoPi;
-      const float Xs = phi * (float)R.resolution.x / kTwoPi;
-      const float ys = o.y + (tca - back * inv_dxz) * d.y;
-      const float Ys = ((ys - R.pos.y) / R.size.y + 0.5f) * (float)R.resolution.y;
-      const float pe = bilinear_p(R, Xs, Ys);
-#pragma unroll
-      for (int k = 0; k < K; ++k) g[k] -= e * pe * out * b.d[k] / w;
-      return;
-    }
-    const float sx = (float)R.resolution.x / kTwoPi, sy = (float)R.resolution.y / R.size.y;
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const float px = origin.x.d[k] + t * rd.x.d[k], py = origin.y.d[k] + t * rd.y.d[k],
-                  pz = origin.z.d[k] + t * rd.z.d[k];
-      dt[k] = -(x * px + z * pz) / den;
-      const float qx = px + dt[k] * d.x, qy = py + dt[k] * d.y, qz = pz + dt[k] * d.z;
-      dY[k] = qy * sy;
-      dX[k] = (x * qz - z * qx) / rr * sx;
-    }
+    band = !(den * den > kGrazing * kGrazing * (rr * dxz2));
+  }
+  if (band) {
+    // Silhouette band: rays whose impact parameter b (distance of the
+    // ray's horizontal line from the axis) lies within w of the radius
+    // (|cos incidence| < kGrazing).  Their interior derivative grows as
+    // 1/cos(incidence) and is not summed; across the band it integrates
+    // to rho e v (P(silhouette) - P(inner band edge)), and the boundary
+    // term of rays crossing the silhouette is -rho e v P(silhouette), so
+    // together the band contributes -rho e v P(inner band edge), with
+    // v = d|b|/dtheta and rho ~ (rays in the band) / w.  P is taken where
+    // this ray's line would meet the cylinder with impact parameter R - w.
+    const float radius = R.size.x;
+    const float w = radius * (1.0f - sqrtf(1.0f - kGrazing * kGrazing));
+    const float inv_dxz = rsqrtf(dxz2);
+    const float ox = o.x - R.pos.x, oz = o.z - R.pos.z;
+    const float b = (ox * d.z - oz * d.x) * inv_dxz;
+    const float out = b >= 0.0f ? 1.0f : -1.0f;
+    const float hx = d.x * inv_dxz, hz = d.z * inv_dxz;  // horizontal unit direction
+    const float tca = -(ox * d.x + oz * d.z) / dxz2;
+    const float cx = o.x + tca * d.x - R.pos.x, cz = o.z + tca * d.z - R.pos.z;  // closest approach
+    const float cl = sqrtf(cx * cx + cz * cz);
+    const float ux = cl > 0.0f ? cx / cl : -hz, uz = cl > 0.0f ? cz / cl : hx;
+    const float back = radius * kGrazing;  // sqrt(R^2 - (R - w)^2)
+    const float ex = (radius - w) * ux - back * hx, ez = (radius - w) * uz - back * hz;
+    float phi = atan2f(ez, ex);
+    if (phi < 0.0f) phi += kTwoPi;
+    const float Xs = phi * (float)R.resolution.x / kTwoPi;
+    const float ys = o.y + (tca - back * inv_dxz) * d.y;
+    const float Ys = ((ys - R.pos.y) / R.size.y + 0.5f) * (float)R.resolution.y;
+    const float pe = bilinear_p(R, Xs, Ys);
+    // b = (ox d.z - oz d.x) / |d_xz|
+    const float bbar = -e * pe * out / w;
+    const float bl = bbar * inv_dxz;
+    obar = make_float3(bl * d.z, 0.0f, -bl * d.x);
+    rdbar = make_float3(-bl * (oz + b * hx), 0.0f, bl * (ox - b * hz));
   } else {
-    const float3 N = qm::cross(R.ab, R.ac);
-    const float nd = qm::dot(N, d), nn = qm::dot(N, N);
-    if (!(fabsf(nd) > kGrazing * sqrtf(nn))) return;  // grazing on a plane: no boundary, detached
-    const float3 abs_ = qm::mul(qm::cross(R.ac, N), 1.0f / nn), acs = qm::mul(qm::cross(N, R.ab), 1.0f / nn);
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      const float3 dox = make_float3(origin.x.d[k], origin.y.d[k], origin.z.d[k]);
-      const float3 ddx = make_float3(rd.x.d[k], rd.y.d[k], rd.z.d[k]);
-      dt[k] = -(qm::dot(N, dox) + t * qm::dot(N, ddx)) / nd;
-      const float3 q = make_float3(dox.x + t * ddx.x + dt[k] * d.x, dox.y + t * ddx.y + dt[k] * d.y,
-                                   dox.z + t * ddx.z + dt[k] * d.z);
-      dY[k] = qm::dot(q, abs_) * (float)R.resolution.y;
-      dX[k] = qm::dot(q, acs) * (float)R.resolution.x;
+    // bilinear P at the deposit position (as the forward's splat)
+    const float X = v * (float)R.resolution.x, Y = u * (float)R.resolution.y;
+    const float xs = X - 0.5f, ys = Y - 0.5f;
+    const Quad q = sample_quad(R, xs, ys);
+    const float pb = bilinear(q);
+    float xbar = e * ((1 - q.fy) * (q.p10 - q.p00) + q.fy * (q.p11 - q.p01));
+    float ybar = e * ((1 - q.fx) * (q.p01 - q.p00) + q.fx * (q.p11 - q.p10));
+    // Image edges (rows of both receivers, columns of a rectangle): rays
+    // within kEdgeBand pixels of an edge estimate the boundary term -rho e P
+    // (outward pixel velocity) of rays leaving or entering across it, with P
+    // taken on the edge itself (half of an edge deposit falls outside).
+    const float by = kEdgeBand;
+    const float H = (float)R.resolution.y, W = (float)R.resolution.x;
+    if (Y < by) ybar += e * bilinear_p(R, X, 0.0f) / by;
+    if (H - Y < by) ybar -= e * bilinear_p(R, X, H) / by;
+    if (R.type == 0) {
+      if (X < by) xbar += e * bilinear_p(R, 0.0f, Y) / by;
+      if (W - X < by) xbar -= e * bilinear_p(R, W, Y) / by;
     }
-  }
-#pragma unroll
-  for (int k = 0; k < K; ++k) {
-    const float de = (sgn * c.d[k] * eta + fabsf(c.v) * deta * dt[k]) * T.factor;
-    g[k] += e * (dpx * dX[k] + dpy * dY[k]) + pb * de;
-  }
-  // Image edges (rows of both receivers, columns of a rectangle): rays within
-  // kEdgeBand pixels of an edge estimate the boundary term -rho e P
-  // (outward pixel velocity) of rays leaving or entering across it, with P
-  // taken on the edge itself (half of an edge deposit falls outside).
-  const float by = kEdgeBand;
-  const float H = (float)R.resolution.y, W = (float)R.resolution.x;
-  if (Y < by) {
-    const float pe = bilinear_p(R, X, 0.0f);
-    for (int k = 0; k < K; ++k) g[k] += e * pe * dY[k] / by;
-  }
-  if (H - Y < by) {
-    const float pe = bilinear_p(R, X, H);
-    for (int k = 0; k < K; ++k) g[k] -= e * pe * dY[k] / by;
-  }
-  if (R.type == 0) {
-    if (X < by) {
-      const float pe = bilinear_p(R, 0.0f, Y);
-      for (int k = 0; k < K; ++k) g[k] += e * pe * dX[k] / by;
+    // e = |c| eta(t) factor
+    const float pf = pb * T.factor;
+    cbar = pf * sgn * eta;
+    float tbar = pf * fabsf(c) * deta;
+    // The hit point q = o + t rd, kept on the surface by dt = -(m . (do + t drd)) / (m . rd), m its normal.
+    float3 qbar, m;
+    float md;
+    if (R.type == 1) {
+      const float a = __fdividef(xbar * ((float)R.resolution.x * (1.0f / kTwoPi)), rr);
+      qbar = make_float3(-a * z, ybar * ((float)R.resolution.y * R.rcp_height), a * x);
+      m = make_float3(x, 0.0f, z);
+      md = den;
+    } else {
+      const float3 N = qm::cross(R.ab, R.ac);
+      const float nd = qm::dot(N, d), nn = qm::dot(N, N);
+      if (!(fabsf(nd) > kGrazing * sqrtf(nn))) return;  // grazing on a plane: no boundary, detached
+      const float3 abs_ = qm::mul(qm::cross(R.ac, N), 1.0f / nn), acs = qm::mul(qm::cross(N, R.ab), 1.0f / nn);
+      qbar = axpy(ybar * H, abs_, qm::mul(acs, xbar * W));
+      m = N;
+      md = nd;
     }
-    if (W - X < by) {
-      const float pe = bilinear_p(R, W, Y);
-      for (int k = 0; k < K; ++k) g[k] -= e * pe * dX[k] / by;
-    }
+    tbar += qm::dot(qbar, d);
+    obar = axpy(-__fdividef(tbar, md), m, qbar);
+    rdbar = make_float3(t * obar.x, t * obar.y, t * obar.z);
   }
+  add_outer(sum, obar, fd.local);
+  if (fd.identity) return;  // the slope-error frame does not turn
+  // rd = in - 2 (np . in) np and c = -(np . in) (np is a unit vector; rd keeps
+  // in's length, so its normalisation has no derivative), then np = slope / |slope|.
+  const float rn = qm::dot(rdbar, np);
+  const float3 npbar = axpy(-2.0f * rn - cbar, in, qm::mul(rdbar, -2.0f * c0.v));
+  const float il = rsqrtf(dot(slope, slope).v);
+  const float3 wbar = qm::mul(axpy(-qm::dot(npbar, np), np, npbar), il);
+  // slope = pert.x u + pert.y n + pert.z v with, for n = (s sin psi, n.y,
+  // s cos psi), u = (cos psi, 0, -sin psi) and v = (n.y sin psi, -s, n.y cos psi).
+  const float sn = -fd.u.z, cs = fd.u.x, s = -fd.v.y;
+  const float along = wbar.x * sn + wbar.z * cs, across = wbar.x * cs - wbar.z * sn;
+  const float psibar = __fdividef(pert.z * fd.n.y * across - pert.x * along, s), sbar = -pert.z * wbar.y;
+  const float3 nbar = make_float3(pert.y * wbar.x + psibar * cs + sbar * sn, pert.y * wbar.y + pert.z * along,
+                                  pert.y * wbar.z - psibar * sn + sbar * cs);
+  add_outer(sum, nbar, fd.local_normal);
 }
 
-
-// Facet window of the adjoint, per warp (as the trace kernel's): the
-// FacetDual of 32 consecutive facets, one per lane, stored component-major so
-// that lanes reading different slots touch different banks.
+// Facet window of the adjoint, per warp (as the trace kernel's): 32
+// consecutive facets, one per lane, stored component-major so that lanes
+// reading different slots touch different banks; and the queue of recorded
+// hits (window slot, light) waiting for a full warp.
 #ifndef QM_BWD_THREADS
 #define QM_BWD_THREADS 32
 #endif
@@ -366,35 +464,30 @@ __device__ __forceinline__ void ray_adjoint(const DevTask& T, const DevReceiver&
 #define QM_BWD_MIN_BLOCKS 20
 #endif
 constexpr int kBwdThreads = QM_BWD_THREADS;
-constexpr int kDual3Words = 3 * (1 + K);
+constexpr int kFacetFloats = 18;
 struct AdjointWindow {
-  float origin[kDual3Words][kBwdThreads];
-  float frame[3 * kDual3Words][kBwdThreads];  // u, n, v
+  float value[kFacetFloats][kBwdThreads];
   int g0[kBwdThreads], g1[kBwdThreads], identity[kBwdThreads];
+  int slot[2 * kBwdThreads], light[2 * kBwdThreads];
+  ChunkConstants shared[kBwdThreads / 32];
 };
 
-__device__ __forceinline__ void put_dual3(float (*dst)[kBwdThreads], int slot, const Dual3& a) {
-  const Dual* c[3] = {&a.x, &a.y, &a.z};
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    dst[i * (1 + K)][slot] = c[i]->v;
-#pragma unroll
-    for (int k = 0; k < K; ++k) dst[i * (1 + K) + 1 + k][slot] = c[i]->d[k];
-  }
+__device__ __forceinline__ void put3(AdjointWindow& w, int first, int slot, float3 a) {
+  w.value[first][slot] = a.x;
+  w.value[first + 1][slot] = a.y;
+  w.value[first + 2][slot] = a.z;
+}
+__device__ __forceinline__ float3 get3(const AdjointWindow& w, int first, int slot) {
+  return make_float3(w.value[first][slot], w.value[first + 1][slot], w.value[first + 2][slot]);
 }
 
-__device__ __forceinline__ Dual3 get_dual3(const float (*src)[kBwdThreads], int slot) {
-  Dual3 a;
-  Dual* c[3] = {&a.x, &a.y, &a.z};
-#pragma unroll
-  for (int i = 0; i < 3; ++i) {
-    c[i]->v = src[i * (1 + K)][slot];
-#pragma unroll
-    for (int k = 0; k < K; ++k) c[i]->d[k] = src[i * (1 + K) + 1 + k][slot];
-  }
-  return a;
-}
-
+// Bound by instruction issue (69 % of slots; 13.4 warp instructions a ray).
+// Run backwards a ray costs its value chain, one sweep of vector adjoints and
+// 18 multiply-adds into the frame sums, against four tangents through every
+// operation (33 warp instructions a ray); the queue gives every sweep 32 hits
+// where a chunk's iterations hold 22 on the benchmark field.  462 M rays, 32
+// lights per facet: 17.9 -> 7.8 ms (11.7 of it before the shared constants and
+// the four-pixel read); 256 M rays, 4 lights: 11.9 -> 6.6.
 __global__ void __launch_bounds__(kBwdThreads, QM_BWD_MIN_BLOCKS) diff_backward_kernel(BackwardParams p) {
   __shared__ AdjointWindow win;
   const int lane = threadIdx.x & 31;
@@ -407,53 +500,80 @@ __global__ void __launch_bounds__(kBwdThreads, QM_BWD_MIN_BLOCKS) diff_backward_
   const int r0 = (int)(chunk - __ldg(p.chunk_prefix + t)) * kChunk;
   const DevTask& T = p.tasks[t];
   const DiffTask& DT = p.dtasks[t];
-  const DevReceiver& R = p.receivers[T.receiver];
+  if (lane == 0) {
+    ChunkConstants& c = win.shared[threadIdx.x >> 5];
+    c.R = p.receivers[T.receiver];
+    c.samples = T.samples;
+    c.perturbations = T.perturbations;
+    c.factor = T.factor;
+  }
   const int r_end = T.num_facets * nl;
   const int iters = min(kChunkIters, (r_end - r0 + 31) >> 5);
   int f = (r0 + lane) / nl;
   int l = (r0 + lane) - f * nl;
-  float g[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k) g[k] = 0.0f;
+  FrameSum sum{};
   int base = 0;
   bool filled = false;  // warp-uniform
+  int queued = 0;       // warp-uniform, below 32 between iterations
+  int* q_slot = win.slot + 2 * wbase;
+  int* q_light = win.light + 2 * wbase;
+  // Runs the last n <= 32 queued hits, one per lane.
+  auto run = [&](int n) {
+    __syncwarp();
+    if (lane < n) {
+      const int slot = q_slot[queued - n + lane], light = q_light[queued - n + lane];
+      Facet fd;
+      fd.origin = get3(win, 0, slot);
+      fd.u = get3(win, 3, slot);
+      fd.n = get3(win, 6, slot);
+      fd.v = get3(win, 9, slot);
+      fd.local = get3(win, 12, slot);
+      fd.local_normal = get3(win, 15, slot);
+      fd.identity = win.identity[slot] != 0;
+      fd.g0 = win.g0[slot];
+      fd.g1 = win.g1[slot];
+      ray_adjoint(win.shared[threadIdx.x >> 5], fd, light, sum);
+    }
+    queued -= n;
+    __syncwarp();
+  };
+  unsigned words = 0;  // lane i: hit bits of iteration 32 (it / 32) + i
   for (int it = 0; it < iters; ++it) {
-    const bool active = r0 + it * 32 + lane < r_end;
-    const unsigned bits = __ldg(p.hit_bits + warp * kChunkIters + it);
+    if ((it & 31) == 0) words = it + lane < iters ? __ldg(p.hit_bits + warp * kChunkIters + it + lane) : 0u;
+    const unsigned bits = __shfl_sync(0xffffffffu, words, it & 31);
+    const bool hit = r0 + it * 32 + lane < r_end && ((bits >> lane) & 1u);
     // The facets of an iteration lie within 32 of lane 0's (see the trace
-    // kernel); refill the window when a lane with a hit needs one past it.
+    // kernel); refill the window when a lane with a hit needs one past it,
+    // after the hits that are waiting with the present one.
     const int f0 = __shfl_sync(0xffffffffu, f, 0);
-    const bool hit = active && ((bits >> lane) & 1u);
     if (__any_sync(0xffffffffu, hit && (!filled || f - base >= 32))) {
+      if (queued > 0) run(queued);
       __syncwarp();
       base = f0;
       filled = true;
       const int fw = base + lane;
       if (fw < T.num_facets) {
-        const FacetDual fd = facet_dual(T, DT, fw);
+        const Facet fd = make_facet(T, DT, fw);
         const int slot = wbase + lane;
-        put_dual3(win.origin, slot, fd.origin);
-        put_dual3(win.frame, slot, fd.pframe.u);
-        put_dual3(win.frame + kDual3Words, slot, fd.pframe.n);
-        put_dual3(win.frame + 2 * kDual3Words, slot, fd.pframe.v);
+        put3(win, 0, slot, fd.origin);
+        put3(win, 3, slot, fd.u);
+        put3(win, 6, slot, fd.n);
+        put3(win, 9, slot, fd.v);
+        put3(win, 12, slot, fd.local);
+        put3(win, 15, slot, fd.local_normal);
         win.g0[slot] = fd.g0;
         win.g1[slot] = fd.g1;
-        win.identity[slot] = fd.pframe.identity ? 1 : 0;
+        win.identity[slot] = fd.identity ? 1 : 0;
       }
-      __syncwarp();
     }
+    const unsigned hits = __ballot_sync(0xffffffffu, hit);
     if (hit) {
-      const int slot = wbase + (f - base);
-      FacetDual fd;
-      fd.origin = get_dual3(win.origin, slot);
-      fd.pframe.u = get_dual3(win.frame, slot);
-      fd.pframe.n = get_dual3(win.frame + kDual3Words, slot);
-      fd.pframe.v = get_dual3(win.frame + 2 * kDual3Words, slot);
-      fd.pframe.identity = win.identity[slot] != 0;
-      fd.g0 = win.g0[slot];
-      fd.g1 = win.g1[slot];
-      ray_adjoint(T, R, fd, p.light_begin + l, g);
+      const int k = queued + __popc(hits & ((1u << lane) - 1u));
+      q_slot[k] = wbase + (f - base);
+      q_light[k] = p.light_begin + l;
     }
+    queued += __popc(hits);
+    if (queued >= 32) run(32);
     f += p.lights_q32;
     l += p.lights_r32;
     if (l >= nl) {
@@ -461,9 +581,16 @@ __global__ void __launch_bounds__(kBwdThreads, QM_BWD_MIN_BLOCKS) diff_backward_
       ++f;
     }
   }
+  if (queued > 0) run(queued);
+  // d(axes)/d(parameters) of the heliostat's facet frame; constant axes when
+  // the frame is the identity.
+  if (DT.identity) return;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    double s = g[k];
+    const float3 du = make_float3(DT.u.x.d[k], DT.u.y.d[k], DT.u.z.d[k]);
+    const float3 dn = make_float3(DT.fn.x.d[k], DT.fn.y.d[k], DT.fn.z.d[k]);
+    const float3 dv = make_float3(DT.v.x.d[k], DT.v.y.d[k], DT.v.z.d[k]);
+    double s = qm::dot(sum.u, du) + qm::dot(sum.n, dn) + qm::dot(sum.v, dv);
     for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
     if (lane == 0 && s != 0.0) atomicAdd(p.grad + (size_t)T.power_slot * K + k, s);
   }

@@ -11,19 +11,22 @@ namespace qm {
 
 constexpr int kDiffParams = 4;  // per heliostat: aim offset u, v (m); normal offset u, v (rad)
 
-// A float and its derivatives with respect to one heliostat's parameters.
-struct Dual {
+// A float and its derivatives with respect to N parameters (0: the value
+// alone, by the same operations).
+template <int N>
+struct DualT {
   float v;
-  float d[kDiffParams];
+  float d[N > 0 ? N : 1];
 };
-struct Dual3 {
-  Dual x, y, z;
+template <int N>
+struct Dual3T {
+  DualT<N> x, y, z;
 };
 
 // Per task: the heliostat normal and its facet frame as functions of the
 // heliostat's parameters (value + tangents), for the adjoint.
 struct DiffTask {
-  Dual3 n, u, fn, v;  // normal; frame (u, n, v) of the facet transform
+  Dual3T<kDiffParams> n, u, fn, v;  // normal; frame (u, n, v) of the facet transform
   int identity;
 };
 
