@@ -38,52 +38,29 @@ float3 sun_of(const float* dirs, int k) {
   return d;
 }
 
-qm::SunFrame sun_frame(float3 sun) {
-  // Frame of -sun_dir, as the plain path builds it.
-  const qm::Frame f = qm::make_frame(qm::neg(sun), false);
-  qm::SunFrame s;
-  s.u = f.u;
-  s.n = f.n;
-  s.v = f.v;
-  s.identity = f.identity ? 1 : 0;
-  return s;
-}
-
 }  // namespace
 
 namespace qrt {
 
-void batch_prepare(qmcrt_batch* b, cudaStream_t st) {
-  for (size_t k = 0; k < b->inst.size(); ++k) {
-    const auto& I = b->inst[k];
-    const int H = (int)I.scene->model.heliostats.size();
-    float3 axis;
-    float tan_world;
-    sun_cone(I.sun, I.scene->sun_shape_tan, axis, tan_world);
-    const float block_theta = tan_world < 0.0f || I.scene->slope_angle < 0.0f
-                                  ? -1.0f
-                                  : std::atan(tan_world) + 2.0f * I.scene->slope_angle;
-    for (int h = 0; h < H; ++h) {
-      qm::PrepItem& it = b->items[I.task_base + h];
-      it.sun_dir = I.sun;
-      it.shadow_axis = axis;
-      it.shadow_tan = tan_world;
-      it.block_theta = block_theta;
-    }
-  }
-  cuda_check(cudaMemcpyAsync(b->d_tasks.p, b->tasks.data(), b->tasks.size() * sizeof(qm::DevTask),
-                             cudaMemcpyHostToDevice, st),
-             "task upload");
-  cuda_check(cudaMemcpyAsync(b->d_items.p, b->items.data(), b->items.size() * sizeof(qm::PrepItem),
-                             cudaMemcpyHostToDevice, st),
-             "prep upload");
-  cuda_check(qm::launch_prep(b->d_items.as<qm::PrepItem>(), (int)b->items.size(), b->d_tasks.as<qm::DevTask>(), st),
-             "prep kernel");
-  int max_sub = 0;
-  for (const auto& it : b->items) max_sub = std::max(max_sub, it.num_sub);
-  cuda_check(qm::launch_shadow_flags(b->d_items.as<qm::PrepItem>(), (int)b->items.size(), max_sub,
-                                     b->d_tasks.as<qm::DevTask>(), b->d_grids.as<qm::DevGrid>(), st),
-             "shadow flags");
+qm::PrepInputs prep_inputs(const qmcrt_batch* b, const float4* params) {
+  qm::PrepInputs p{};
+  p.items = b->d_items.as<qm::PrepItem>();
+  p.n = (int)b->items.size();
+  p.tasks = b->d_tasks.as<qm::DevTask>();
+  p.suns = b->d_suns.as<qm::SunParams>();
+  p.params = params;
+  return p;
+}
+
+void batch_prepare(qmcrt_batch* b, cudaStream_t st, const float4* params) {
+  std::vector<qm::SunParams> suns;
+  for (const auto& I : b->inst) suns.push_back(sun_params(I.sun, I.scene->sun_shape_tan, I.scene->slope_angle));
+  b->d_suns.alloc(suns.size() * sizeof(qm::SunParams));
+  cuda_check(cudaMemcpyAsync(b->d_suns.p, suns.data(), suns.size() * sizeof(qm::SunParams), cudaMemcpyHostToDevice, st),
+             "sun upload");
+  const qm::PrepInputs in = prep_inputs(b, params);
+  cuda_check(qm::launch_prep(in, st), "prep kernel");
+  cuda_check(qm::launch_shadow_flags(in, b->max_sub, b->d_grids.as<qm::DevGrid>(), st), "shadow flags");
   std::vector<qm::PoolRotation> rot(b->inst.size());
   int max_out = 0;
   for (size_t k = 0; k < b->inst.size(); ++k) {
@@ -96,7 +73,9 @@ void batch_prepare(qmcrt_batch* b, cudaStream_t st) {
     rot[k].sun = sun_frame(I.sun);
     max_out = std::max(max_out, rot[k].n_out);
   }
-  upload(b->d_rot, rot);
+  b->d_rot.alloc(rot.size() * sizeof(qm::PoolRotation));
+  cuda_check(cudaMemcpyAsync(b->d_rot.p, rot.data(), rot.size() * sizeof(qm::PoolRotation), cudaMemcpyHostToDevice, st),
+             "pool rotation upload");
   for (size_t k0 = 0; k0 < rot.size(); k0 += 65535) {
     const int n = (int)std::min<size_t>(65535, rot.size() - k0);
     cuda_check(qm::launch_rotate_pools(b->d_rot.as<qm::PoolRotation>() + k0, n, max_out, st), "pool rotation");
@@ -225,6 +204,9 @@ int qmcrt_batch_create(qmcrt_scene* const* scenes, int n_scenes, const int* scen
         b->tasks.push_back(t);  // samples pointer set below; normal and frames by the prep kernel
         qm::PrepItem it{};
         it.task = I.task_base + h;
+        it.sun = k;
+        it.param = h;
+        b->max_sub = std::max(b->max_sub, hm.num_sub);
         it.num_sub = hm.num_sub;
         it.sub_first = hm.sub_begin;
         it.focus = hm.focus;
@@ -274,8 +256,8 @@ int qmcrt_batch_create(qmcrt_scene* const* scenes, int n_scenes, const int* scen
     }
     upload(b->d_grids, b->grids);
     upload(b->d_receivers, b->receivers);
-    b->d_tasks.alloc(b->tasks.size() * sizeof(qm::DevTask));
-    b->d_items.alloc(b->items.size() * sizeof(qm::PrepItem));
+    upload(b->d_tasks, b->tasks);
+    upload(b->d_items, b->items);
     b->light_begin = 0;
     b->light_end = b->max_lights;
     batch_prepare(b.get(), 0);

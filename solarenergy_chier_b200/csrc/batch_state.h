@@ -23,11 +23,12 @@ struct qmcrt_batch {
   std::vector<qm::DevReceiver> receivers;
   std::vector<qm::DevTask> tasks;
   std::vector<qm::PrepItem> items;
-  qrt::DBuf d_grids, d_receivers, d_tasks, d_prefix, d_items, d_rot;
+  qrt::DBuf d_grids, d_receivers, d_tasks, d_prefix, d_items, d_suns, d_rot;
   qrt::DBuf d_bound, d_hsub, d_subv, d_verts, d_sub_free, d_sub_cand, d_sub_frames;  // per instance-grid slices
   qrt::DBuf d_images, d_power, d_diag, d_pools;
   qrt::DBuf d_chunk_power;  // per-chunk FP64 power partials of a launch (sized with the chunk prefix)
   qrt::DBuf d_work;         // work counter of persistent flux launches
+  int max_sub = 0;  // most sub-heliostats of any heliostat
   int light_begin = 0, light_end = 0, max_lights = 0;
   long long total_chunks = -1;  // for the current light range; -1 = prefix not built
   int chunk_iters = qm::kChunkIters;  // warp-chunk iterations of the prefix
@@ -52,7 +53,7 @@ struct qmcrt_batch {
     cudaSetDevice(device);
     cudaDeviceSynchronize();
     drop_graph();
-    for (qrt::DBuf* b : {&d_grids, &d_receivers, &d_tasks, &d_prefix, &d_items, &d_rot, &d_bound, &d_hsub, &d_subv,
+    for (qrt::DBuf* b : {&d_grids, &d_receivers, &d_tasks, &d_prefix, &d_items, &d_suns, &d_rot, &d_bound, &d_hsub, &d_subv,
                     &d_verts, &d_sub_free, &d_sub_cand, &d_sub_frames, &d_images, &d_power, &d_diag, &d_pools,
                     &d_chunk_power, &d_work})
       b->release();
@@ -62,9 +63,11 @@ struct qmcrt_batch {
 
 namespace qrt {
 
-// Uploads the tasks and preparation items and prepares every instance for
-// its sun on the device (normals, frames, parallelograms, records, pools).
-void batch_prepare(qmcrt_batch* b, cudaStream_t st);
+// Inputs of the preparation kernels (params: per heliostat of one scene, or NULL).
+qm::PrepInputs prep_inputs(const qmcrt_batch* b, const float4* params);
+// Prepares every instance for its sun on the device (normals, frames,
+// parallelograms, records, walk codes, pools); returns when that is done.
+void batch_prepare(qmcrt_batch* b, cudaStream_t st, const float4* params = nullptr);
 // Chunk prefix of the tasks for the current light range.
 void batch_build_prefix(qmcrt_batch* b);
 // One trace launch over the tasks' warp chunks [chunk_begin, chunk_end)

@@ -56,42 +56,23 @@ using qm::DevGrid;
 using qm::DevReceiver;
 using qm::DevTask;
 
-// Sun-dependent data of one grid: per heliostat its traversal record and
-// (first sub-heliostat, count, lattice rows, lattice columns), and per
-// sub-heliostat its parallelogram as A, B - A, C - A.
-void grid_sun_data(const qm::SceneModel& m, const qm::GridModel& g, std::vector<float4>& bound,
-                   std::vector<int4>& hsub, std::vector<float4>& subv) {
-  bound.assign(5 * (size_t)g.num_heliostats, float4{});
-  hsub.assign(g.num_heliostats, int4{});
-  for (int i = 0; i < g.num_heliostats; ++i) {
-    const qm::HeliostatModel& h = m.heliostats[g.start_heliostat + i];
-    int2 rc;
-    qm::heliostat_record(g.sub_vertices.data() + 3 * (size_t)h.sub_begin, h.num_sub, h.row_col, h.pos, h.normal,
-                         &bound[5 * (size_t)i], &rc);
-    hsub[i] = make_int4(h.sub_begin, h.num_sub, rc.x, rc.y);
-  }
-  subv.assign(3 * (size_t)g.num_subheliostats, float4{});
-  for (int sidx = 0; sidx < g.num_subheliostats; ++sidx) {
-    const float3 B = g.sub_vertices[3 * sidx], A = g.sub_vertices[3 * sidx + 1], C = g.sub_vertices[3 * sidx + 2];
-    const float3 ab = qm::sub(B, A), ac = qm::sub(C, A);
-    subv[3 * sidx] = make_float4(A.x, A.y, A.z, ab.x);
-    subv[3 * sidx + 1] = make_float4(ab.y, ab.z, ac.x, ac.y);
-    subv[3 * sidx + 2] = make_float4(ac.z, 0.f, 0.f, 0.f);
-  }
+qm::SunFrame sun_frame(float3 sun_dir) {
+  // -sun_dir (QuasiMonteCarloRayTracer::generateSunrayArgument feeds
+  // -sunray_direction to local2world_rotate per ray; the frame is constant).
+  const qm::Frame f = qm::make_frame(qm::neg(sun_dir), false);
+  qm::SunFrame s;
+  s.u = f.u;
+  s.n = f.n;
+  s.v = f.v;
+  s.identity = f.identity ? 1 : 0;
+  return s;
 }
 
-// Sun frame and per-heliostat task templates (both depend on the sun).
+// The sun-independent fields of every heliostat's task, and what the device
+// prepares the others from.
 void build_templates(qmcrt_scene* s) {
   const qm::SceneModel& m = s->model;
   const qm::SceneConfig& cfg = m.config;
-  // Sun frame of -sun_dir (QuasiMonteCarloRayTracer::generateSunrayArgument feeds
-  // -sunray_direction to local2world_rotate per ray; the frame is constant).
-  qm::Frame f = qm::make_frame(qm::neg(cfg.sun_dir), false);
-  s->sun.u = f.u;
-  s->sun.n = f.n;
-  s->sun.v = f.v;
-  s->sun.identity = f.identity ? 1 : 0;
-
   s->templates.assign(m.heliostats.size(), DevTask{});
   for (size_t i = 0; i < m.heliostats.size(); ++i) {
     const auto& h = m.heliostats[i];
@@ -114,12 +95,6 @@ void build_templates(qmcrt_scene* s) {
     t.sub_length = h.sub_length;
     t.size = h.size;
     t.pos = h.pos;
-    t.normal = h.normal;
-    qm::Frame hf = qm::make_frame(h.normal, h.type == 1);
-    t.fu = hf.u;
-    t.fn = hf.n;
-    t.fv = hf.v;
-    t.frame_identity = hf.identity ? 1 : 0;
     if (h.type == 1) {
       const float3* base = s->d_local.as<float3>() + s->local_base[i];
       t.local_centers = base;
@@ -131,7 +106,57 @@ void build_templates(qmcrt_scene* s) {
     t.pool_size = s->pool_size;
     s->templates[i] = t;
   }
-  s->cache_valid = false;
+  upload(s->d_templates, s->templates);
+  std::vector<qm::PrepItem> items(m.heliostats.size());
+  s->max_sub = 0;
+  for (size_t i = 0; i < items.size(); ++i) {
+    const auto& h = m.heliostats[i];
+    const GridBufs& gb = *s->grid_bufs[h.grid];
+    qm::PrepItem& it = items[i];
+    it.task = (int)i;
+    it.num_sub = h.num_sub;
+    it.sub_first = h.sub_begin;
+    it.focus = h.focus;
+    it.sub_free = gb.sub_free.as<int>() + h.sub_begin;
+    it.sub_cand = gb.sub_cand.as<int>() + (size_t)h.sub_begin * qm::kMaxCandidates;
+    it.sub_frames = gb.sub_frames.as<float4>() + 6 * (size_t)h.sub_begin;
+    it.verts = gb.verts.as<float3>() + 3 * (size_t)h.sub_begin;
+    it.subv = gb.subv.as<float4>() + 3 * (size_t)h.sub_begin;
+    const int own = (int)i - m.grids[h.grid].start_heliostat;
+    it.bound = gb.bound.as<float4>() + 5 * (size_t)own;
+    it.hsub = gb.hsub.as<int4>() + own;
+    s->max_sub = std::max(s->max_sub, h.num_sub);
+  }
+  upload(s->d_items, items);
+}
+
+// Queues the preparation of every heliostat for the configuration's sun
+// (normals, facet frames, parallelograms, traversal records): the
+// sun-dependent half of SceneProcessor::processScene on the device, equal to
+// the host's bit for bit.
+qm::PrepInputs sun_inputs(qmcrt_scene* s) {
+  const qm::SunParams sun = sun_params(s->model.config.sun_dir, s->sun_shape_tan, s->slope_angle);
+  s->d_sun.alloc(sizeof(sun));
+  cuda_check(cudaMemcpyAsync(s->d_sun.p, &sun, sizeof(sun), cudaMemcpyHostToDevice, 0), "sun upload");
+  qm::PrepInputs p{};
+  p.items = s->d_items.as<qm::PrepItem>();
+  p.n = (int)s->templates.size();
+  p.tasks = s->d_templates.as<DevTask>();
+  p.suns = s->d_sun.as<qm::SunParams>();
+  return p;
+}
+
+void prepare_sun(qmcrt_scene* s) {
+  s->sun = sun_frame(s->model.config.sun_dir);
+  cuda_check(qm::launch_prep(sun_inputs(s), 0), "prep kernel");
+  s->gathered = false;
+}
+
+// The model's normals and vertices for the current sun, for the getters.
+void model_for_sun(const qmcrt_scene* s) {
+  if (!s->model_stale) return;
+  qm::set_sun(const_cast<qmcrt_scene*>(s)->model, s->model.config.sun_dir);
+  s->model_stale = false;
 }
 
 void build_device_scene(qmcrt_scene* s) {
@@ -160,12 +185,12 @@ void build_device_scene(qmcrt_scene* s) {
     }
     upload(gb->ranges, ranges);
     upload(gb->entries, entries);
-    std::vector<float4> bound, subv;
-    std::vector<int4> hsub;
-    grid_sun_data(m, g, bound, hsub, subv);
-    upload(gb->bound, bound);
-    upload(gb->hsub, hsub);
-    upload(gb->subv, subv);
+    // written by the preparation of every sun
+    const size_t helios = std::max(g.num_heliostats, 1), subs = std::max(g.num_subheliostats, 1);
+    gb->bound.alloc(5 * helios * sizeof(float4));
+    gb->hsub.alloc(helios * sizeof(int4));
+    gb->subv.alloc(3 * subs * sizeof(float4));
+    gb->verts.alloc(3 * subs * sizeof(float3));
     // block-free flags start cleared (no skipping) until the pools exist
     upload(gb->sub_free, std::vector<int>(std::max(g.num_subheliostats, 1), 0));
     upload(gb->sub_cand, std::vector<int>((size_t)std::max(g.num_subheliostats, 1) * qm::kMaxCandidates, -1));
@@ -242,7 +267,7 @@ void build_device_scene(qmcrt_scene* s) {
   s->d_samples.alloc((size_t)P * sizeof(float4));
   s->d_perturb.alloc((size_t)P * sizeof(float4));
   s->d_trace_samples.alloc((size_t)(P + cfg.num_per_sunshape_group) * sizeof(float4));
-  s->d_scratch_word.alloc(sizeof(unsigned));
+  s->d_pool_stats.alloc(sizeof(qm::PoolStats));
   s->d_trace_perturb.alloc((size_t)(P + cfg.num_per_sunshape_group) * sizeof(float4));
   {
     std::vector<long long> seg(s->offset_base);
@@ -255,7 +280,7 @@ void build_device_scene(qmcrt_scene* s) {
   cuda_check(cudaMemset(s->d_diag.p, 0, s->d_diag.bytes), "cudaMemset");
 
   build_templates(s);
-  s->cache_valid = false;
+  prepare_sun(s);
 }
 
 void generate_offsets(qmcrt_scene* s, unsigned seed) {
@@ -266,95 +291,66 @@ void generate_offsets(qmcrt_scene* s, unsigned seed) {
   cuda_check(cudaDeviceSynchronize(), "offsets kernel");
 }
 
-// Sun axis and tangent of the largest sun-shape angle in world space, for
-// the shadow-free test, from the tangent `tan_local` of the local pool (the
-// sun frame maps the local y axis to -sun_dir, which may not be unit length;
-// an identity frame leaves samples as they are).
-void sun_cone(float3 sun_dir, float tan_local, float3& axis, float& tan_world) {
+// Sun axis and tangent of the largest sun-shape angle in world space, from
+// the tangent `tan_local` of the local pool (the sun frame maps the local y
+// axis to -sun_dir, which may not be unit length; an identity frame leaves
+// samples as they are).
+qm::SunParams sun_params(float3 sun_dir, float tan_local, float slope_angle) {
+  qm::SunParams p{};
+  p.dir = sun_dir;
   const qm::Frame f = qm::make_frame(qm::neg(sun_dir), false);
   if (f.identity) {
-    axis = make_float3(0.f, 1.f, 0.f);
-    tan_world = tan_local;
-    return;
+    p.shadow_axis = make_float3(0.f, 1.f, 0.f);
+    p.shadow_tan = tan_local;
+  } else {
+    p.shadow_axis = qm::neg(sun_dir);
+    const double len = std::sqrt((double)sun_dir.x * sun_dir.x + (double)sun_dir.y * sun_dir.y +
+                                 (double)sun_dir.z * sun_dir.z);
+    p.shadow_tan = tan_local < 0.0f ? -1.0f : (float)(tan_local / len);
   }
-  axis = qm::neg(sun_dir);
-  const double len = std::sqrt((double)sun_dir.x * sun_dir.x + (double)sun_dir.y * sun_dir.y +
-                               (double)sun_dir.z * sun_dir.z);
-  tan_world = tan_local < 0.0f ? -1.0f : (float)(tan_local / len);
+  p.block_theta =
+      p.shadow_tan < 0.0f || slope_angle < 0.0f ? -1.0f : std::atan(p.shadow_tan) + 2.0f * slope_angle;
+  return p;
 }
 
-// Tangent of the largest angle between a pool direction and the pool's
-// local +y axis, reduced on the device (-1 when some direction has y <= 0:
-// unbounded).
-float pool_tan(qmcrt_scene* s, const DBuf& pool) {
-  cuda_check(cudaMemset(s->d_scratch_word.p, 0, sizeof(unsigned)), "cudaMemset");
-  cuda_check(qm::launch_pool_tan(pool.as<float4>(), s->pool_size, s->d_scratch_word.as<unsigned>(), 0), "pool bound");
-  unsigned bits = 0;
-  cuda_check(cudaMemcpy(&bits, s->d_scratch_word.p, sizeof(unsigned), cudaMemcpyDeviceToHost), "pool bound");
-  float t;
-  std::memcpy(&t, &bits, sizeof(t));
-  return std::isfinite(t) ? t : -1.0f;
+// Largest angles of the pools (PoolStats bits): the tangent of the
+// sun-shape pool's, the slope-error pool's in radians; -1 when some direction
+// has y <= 0 (unbounded).
+void set_pool_bounds(qmcrt_scene* s, const qm::PoolStats& stats) {
+  float t[2];
+  static_assert(sizeof(t) == sizeof(stats.tan_bits), "two floats");
+  std::memcpy(t, stats.tan_bits, sizeof(t));
+  s->sun_shape_tan = std::isfinite(t[0]) ? t[0] : -1.0f;
+  s->slope_angle = std::isfinite(t[1]) ? std::atan(t[1]) : -1.0f;
 }
 
-// Walk-free flags (csrc/shadow.h) for the current sun and pools, computed on
-// the device: per heliostat template for the shadow walks, per sub-heliostat
-// (each grid's sub_free array) for the block walks.  Skipped when neither the
-// sun nor the pools' angular bounds changed since the last computation.
-void update_shadow_flags(qmcrt_scene* s, bool pools_changed) {
-  if (pools_changed || s->sun_shape_tan < -1.5f) {
-    s->sun_shape_tan = pool_tan(s, s->d_samples);
-    const float slope_tan = pool_tan(s, s->d_perturb);
-    s->slope_angle = slope_tan < 0.0f ? -1.0f : std::atan(slope_tan);
-  }
+// Queues the walk codes (csrc/shadow.h) for the current sun and pools: per
+// heliostat template for the shadow walks, per sub-heliostat (each grid's
+// sub_free array) for the block walks.  Skipped when neither the sun nor the
+// pools' angular bounds changed since the last computation.
+void update_walk_codes(qmcrt_scene* s) {
   const float3 sun = s->model.config.sun_dir;
   if (s->flags_valid && sun.x == s->flags_sun.x && sun.y == s->flags_sun.y && sun.z == s->flags_sun.z &&
       s->sun_shape_tan == s->flags_tan && s->slope_angle == s->flags_slope)
     return;
-  float3 axis;
-  float tan_world;
-  sun_cone(sun, s->sun_shape_tan, axis, tan_world);
-  qm::WalkFlagParams p{};
-  upload(s->d_flag_tasks, s->templates);
-  s->d_flag_out.alloc(std::max<size_t>(s->templates.size(), 1) * (1 + qm::kMaxCandidates) * sizeof(int));
-  p.tasks = s->d_flag_tasks.as<DevTask>();
-  p.n = (int)s->templates.size();
-  p.max_sub = 0;
-  for (const auto& h : s->model.heliostats) p.max_sub = std::max(p.max_sub, h.num_sub);
-  p.grids = s->d_grids.as<DevGrid>();
-  p.sun_axis = axis;
-  p.sun_tan = tan_world;
-  p.sun_dir = sun;
-  p.block_theta = tan_world < 0.0f || s->slope_angle < 0.0f ? -1.0f : std::atan(tan_world) + 2.0f * s->slope_angle;
-  const size_t nt = s->templates.size();
-  p.shadow_out = s->d_flag_out.as<int>();
-  p.shadow_cand_out = s->d_flag_out.as<int>() + nt;
-  cuda_check(qm::launch_walk_flags(p, 0), "walk flags");
-  std::vector<int> flags(nt * (1 + qm::kMaxCandidates));
-  if (!flags.empty())
-    cuda_check(cudaMemcpy(flags.data(), s->d_flag_out.p, flags.size() * sizeof(int), cudaMemcpyDeviceToHost),
-               "walk flags");
-  for (size_t i = 0; i < nt; ++i) {
-    s->templates[i].shadow_free = flags[i];
-    for (int k = 0; k < qm::kMaxCandidates; ++k)
-      s->templates[i].shadow_cand[k] = flags[nt + i * qm::kMaxCandidates + k];
-  }
+  cuda_check(qm::launch_shadow_flags(sun_inputs(s), s->max_sub, s->d_grids.as<DevGrid>(), 0), "walk codes");
+  s->gathered = false;
   s->flags_valid = true;
   s->flags_sun = sun;
   s->flags_tan = s->sun_shape_tan;
   s->flags_slope = s->slope_angle;
-  s->cache_valid = false;
 }
 
 // The tracer's copies of the pools (world-space samples, P + L entries);
-// redone after every change of the pools or of the sun, with the
-// shadow-free flags that depend on both.
-void rotate_pool(qmcrt_scene* s, bool pools_changed) {
+// redone after every change of the pools or of the sun, with the walk codes
+// that depend on both.  Returns when the device is done.
+void rotate_pool(qmcrt_scene* s) {
   const int n_out = s->pool_size + s->model.config.num_per_sunshape_group;
   cuda_check(qm::launch_trace_pools(s->d_samples.as<float4>(), s->d_perturb.as<float4>(), s->pool_size, n_out, s->sun,
                                     s->d_trace_samples.as<float4>(), s->d_trace_perturb.as<float4>(), 0),
              "pool rotation");
+  update_walk_codes(s);
   cuda_check(cudaDeviceSynchronize(), "pool rotation");
-  update_shadow_flags(s, pools_changed);
 }
 
 void generate_pool(qmcrt_scene* s, unsigned seed, int sunshape, float half_angle) {
@@ -386,8 +382,15 @@ void generate_pool(qmcrt_scene* s, unsigned seed, int sunshape, float half_angle
     invalid("sunshape must be 0 (Buie) or 1 (pillbox)");
   }
   cuda_check(qm::launch_pool(p, 0), "pool kernel");
-  cuda_check(cudaDeviceSynchronize(), "pool kernel");
-  rotate_pool(s, true);
+  qm::PoolStats* stats = s->d_pool_stats.as<qm::PoolStats>();
+  cuda_check(cudaMemsetAsync(stats, 0, sizeof(qm::PoolStats), 0), "pool bound");
+  cuda_check(qm::launch_pool_stats(reinterpret_cast<const float*>(p.samples), reinterpret_cast<const float*>(p.perturbations), 4,
+                                   s->pool_size, stats, 0),
+             "pool bound");
+  qm::PoolStats found;
+  cuda_check(cudaMemcpy(&found, stats, sizeof(found), cudaMemcpyDeviceToHost), "pool kernel");
+  set_pool_bounds(s, found);
+  rotate_pool(s);
 }
 
 qmcrt_scene* checked(qmcrt_scene* s) {
@@ -407,19 +410,20 @@ void check_heliostat(const qmcrt_scene* s, int id) {
 void ensure_stage(qmcrt_scene* s, size_t n) {
   if (s->stage_done) cuda_check(cudaEventSynchronize(s->stage_done), "cudaEventSynchronize");
   if (n <= s->stage_cap) return;
-  if (s->h_stage) cudaFreeHost(s->h_stage);
+  if (s->h_ids) cudaFreeHost(s->h_ids);
   if (s->h_prefix) cudaFreeHost(s->h_prefix);
-  s->h_stage = nullptr;
+  s->h_ids = nullptr;
   s->h_prefix = nullptr;
+  s->stage_cap = 0;
+  s->cached_ids.clear();
   size_t cap = std::max<size_t>(n, 64);
   alloc_gate("cudaMallocHost");
-  cuda_check(cudaMallocHost((void**)&s->h_stage, cap * sizeof(DevTask)), "cudaMallocHost");
+  cuda_check(cudaMallocHost((void**)&s->h_ids, cap * sizeof(int)), "cudaMallocHost");
   alloc_gate("cudaMallocHost");
   cuda_check(cudaMallocHost((void**)&s->h_prefix, (cap + 1) * sizeof(long long)), "cudaMallocHost");
-  s->d_tasks.alloc(cap * sizeof(DevTask));
+  s->d_ids.alloc(cap * sizeof(int));
   s->d_prefix.alloc((cap + 1) * sizeof(long long));
   s->stage_cap = cap;
-  s->cache_valid = false;
 }
 
 qm::TraceParams base_params(qmcrt_scene* s) {
@@ -519,31 +523,63 @@ long long trace_ids(qmcrt_scene* s, const int* ids, int n, cudaStream_t stream, 
   const int chunk_iters = chunk_iters_for(s->exact, s->shape, out, rays);
   const long long chunk = 32LL * chunk_iters;
   auto chunks_of = [&](int id) { return ((long long)s->templates[id].num_facets * nl + chunk - 1) / chunk; };
-  bool same = s->cache_valid && s->cached_lights == nl && s->cached_chunk == chunk && (int)s->cached_ids.size() == n &&
-              std::equal(ids, ids + n, s->cached_ids.begin());
+  bool consecutive = true;
+  for (int i = 1; i < n; ++i) consecutive = consecutive && ids[i] == ids[0] + i;
   long long total = 0;
-  if (!same) {
-    ensure_stage(s, (size_t)n);
-    s->h_prefix[0] = 0;
-    for (int i = 0; i < n; ++i) {
-      s->h_stage[i] = s->templates[ids[i]];
-      s->h_prefix[i + 1] = s->h_prefix[i] + chunks_of(ids[i]);
-    }
-    cuda_check(cudaMemcpyAsync(s->d_tasks.p, s->h_stage, n * sizeof(DevTask), cudaMemcpyHostToDevice, stream),
-               "task upload");
-    cuda_check(cudaMemcpyAsync(s->d_prefix.p, s->h_prefix, (n + 1) * sizeof(long long), cudaMemcpyHostToDevice, stream),
-               "task upload");
-    if (!s->stage_done) cuda_check(cudaEventCreateWithFlags(&s->stage_done, cudaEventDisableTiming), "cudaEventCreate");
-    cuda_check(cudaEventRecord(s->stage_done, stream), "cudaEventRecord");
-    s->cached_ids.assign(ids, ids + n);
-    s->cached_lights = nl;
-    s->cached_chunk = chunk;
-    s->cache_valid = true;
-  }
   for (int i = 0; i < n; ++i) total += chunks_of(ids[i]);
   qm::TraceParams p = base_params(s);
-  p.tasks = s->d_tasks.as<DevTask>();
-  p.facet_prefix = s->d_prefix.as<long long>();
+  if (n == 1) {
+    // One heliostat, as the reference traces them: its task and its chunk
+    // count lie on the device, so a call uploads nothing.
+    if (s->single_lights != nl || s->single_chunk != chunk) {
+      std::vector<long long> single(2 * s->templates.size(), 0);
+      for (size_t h = 0; h < s->templates.size(); ++h) single[2 * h + 1] = chunks_of((int)h);
+      s->single_lights = -1;
+      s->d_single.alloc(single.size() * sizeof(long long));
+      cuda_check(cudaMemcpyAsync(s->d_single.p, single.data(), single.size() * sizeof(long long), cudaMemcpyHostToDevice,
+                                 stream),
+                 "chunk table");
+      s->single_lights = nl;
+      s->single_chunk = chunk;
+    }
+    p.tasks = s->d_templates.as<DevTask>() + ids[0];
+    p.facet_prefix = s->d_single.as<long long>() + 2 * (size_t)ids[0];
+  } else {
+    const bool listed = (int)s->cached_ids.size() == n && std::equal(ids, ids + n, s->cached_ids.begin());
+    if (!listed || s->cached_lights != nl || s->cached_chunk != chunk) {
+      ensure_stage(s, (size_t)n);
+      s->h_prefix[0] = 0;
+      for (int i = 0; i < n; ++i) s->h_prefix[i + 1] = s->h_prefix[i] + chunks_of(ids[i]);
+      std::copy(ids, ids + n, s->h_ids);
+      s->cached_ids.clear();
+      cuda_check(cudaMemcpyAsync(s->d_prefix.p, s->h_prefix, (n + 1) * sizeof(long long), cudaMemcpyHostToDevice, stream),
+                 "task upload");
+      if (!consecutive)
+        cuda_check(cudaMemcpyAsync(s->d_ids.p, s->h_ids, n * sizeof(int), cudaMemcpyHostToDevice, stream), "task upload");
+      if (!s->stage_done) cuda_check(cudaEventCreateWithFlags(&s->stage_done, cudaEventDisableTiming), "cudaEventCreate");
+      cuda_check(cudaEventRecord(s->stage_done, stream), "cudaEventRecord");
+      s->cached_ids.assign(ids, ids + n);
+      s->cached_lights = nl;
+      s->cached_chunk = chunk;
+      s->gathered = s->gathered && listed;
+    }
+    if (consecutive) {
+      p.tasks = s->d_templates.as<DevTask>() + ids[0];
+    } else {
+      if (s->d_tasks.bytes < s->stage_cap * sizeof(DevTask)) {
+        s->d_tasks.alloc(s->stage_cap * sizeof(DevTask));
+        s->gathered = false;
+      }
+      if (!s->gathered) {
+        cuda_check(qm::launch_gather_tasks(s->d_templates.as<DevTask>(), s->d_ids.as<int>(), n, s->d_tasks.as<DevTask>(),
+                                           stream),
+                   "task gather");
+        s->gathered = true;
+      }
+      p.tasks = s->d_tasks.as<DevTask>();
+    }
+    p.facet_prefix = s->d_prefix.as<long long>();
+  }
   p.num_tasks = n;
   p.total_facets = total;
   p.hit_bits = hit_bits;
@@ -688,6 +724,7 @@ int qmcrt_heliostat_get(const qmcrt_scene* s, int id, int* type, int* grid, int*
   return guarded([&] {
     if (!s) invalid("scene is NULL");
     check_heliostat(s, id);
+    if (normal3) model_for_sun(s);
     const auto& h = s->model.heliostats[id];
     if (type) *type = h.type;
     if (grid) *grid = h.grid;
@@ -730,6 +767,7 @@ int qmcrt_grid_vertices(const qmcrt_scene* s, int id, float* xyz) {
   return guarded([&] {
     if (!s || !xyz) invalid("scene or output is NULL");
     if (id < 0 || id >= (int)s->model.grids.size()) invalid("grid index out of range");
+    model_for_sun(s);
     const auto& g = s->model.grids[id];
     for (size_t i = 0; i < g.sub_vertices.size(); ++i) {
       xyz[3 * i] = g.sub_vertices[i].x;
@@ -745,7 +783,8 @@ int qmcrt_heliostat_facets(qmcrt_scene* s, int id, float* origins, float* normal
     check_heliostat(s, id);
     if (!origins || !normals) invalid("output is NULL");
     DeviceGuard guard(s->device);
-    const DevTask& t = s->templates[id];
+    DevTask t;
+    cuda_check(cudaMemcpy(&t, s->d_templates.as<DevTask>() + id, sizeof(t), cudaMemcpyDeviceToHost), "task readback");
     DBuf o, n;
     o.alloc(std::max<size_t>(t.num_facets, 1) * sizeof(float3));
     n.alloc(std::max<size_t>(t.num_facets, 1) * sizeof(float3));
@@ -764,25 +803,17 @@ int qmcrt_scene_set_sun(qmcrt_scene* s, const float* sun_dir) {
     const float3 d = make_float3(sun_dir[0], sun_dir[1], sun_dir[2]);
     if (!std::isfinite(d.x) || !std::isfinite(d.y) || !std::isfinite(d.z) || (d.x == 0 && d.y == 0 && d.z == 0))
       invalid("sun direction must be finite and non-zero");
-    qm::set_sun(s->model, d);
-    if (s->device < 0) return;
+    if (s->device < 0) {
+      qm::set_sun(s->model, d);
+      return;
+    }
     DeviceGuard guard(s->device);
     cuda_check(cudaDeviceSynchronize(), "set_sun");
-    for (size_t g = 0; g < s->model.grids.size(); ++g) {
-      std::vector<float4> bound, subv;
-      std::vector<int4> hsub;
-      grid_sun_data(s->model, s->model.grids[g], bound, hsub, subv);
-      upload(s->grid_bufs[g]->bound, bound);
-      upload(s->grid_bufs[g]->hsub, hsub);
-      upload(s->grid_bufs[g]->subv, subv);
-      s->grids[g].bound = s->grid_bufs[g]->bound.as<float4>();
-      s->grids[g].hsub = s->grid_bufs[g]->hsub.as<int4>();
-      s->grids[g].subv = s->grid_bufs[g]->subv.as<float4>();
-    }
-    upload(s->d_grids, s->grids);
-    build_templates(s);
+    s->model.config.sun_dir = d;
+    s->model_stale = true;
     s->flags_valid = false;
-    rotate_pool(s, false);
+    prepare_sun(s);
+    rotate_pool(s);
   });
 }
 
@@ -796,30 +827,28 @@ int qmcrt_set_sample_pool(qmcrt_scene* s, const float* dirs, const float* pertur
       invalid("pool shape must match the configuration's groups x lights-per-group");
     DeviceGuard guard(s->device);
     const int n = s->pool_size;
-    // staging for both xyz pools and a counter word after them, kept with the
-    // scene (allocated once)
+    // staging for both xyz pools, kept with the scene (allocated once)
     DBuf& tmp = s->d_pool_stage;
-    const size_t stage_bytes = (size_t)n * 6 * sizeof(float) + sizeof(unsigned);
+    const size_t stage_bytes = (size_t)n * 6 * sizeof(float);
     if (tmp.bytes < stage_bytes) tmp.alloc(stage_bytes);
     float* stage_dirs = tmp.as<float>();
     float* stage_pert = stage_dirs + (size_t)n * 3;
-    unsigned* bad = reinterpret_cast<unsigned*>(stage_pert + (size_t)n * 3);
     const cudaMemcpyKind kind = on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice;
     cuda_check(cudaMemcpy(stage_dirs, dirs, (size_t)n * 3 * sizeof(float), kind), "pool upload");
     cuda_check(cudaMemcpy(stage_pert, perturb, (size_t)n * 3 * sizeof(float), kind), "pool upload");
     // Both pools must hold unit vectors (the tracer normalises the perturbed
     // normal and the reflected ray without a range test); the scene's pools
     // are left as they were when a vector is refused.
-    cuda_check(cudaMemsetAsync(bad, 0, sizeof(unsigned), 0), "pool check");
-    cuda_check(qm::launch_count_non_unit(stage_dirs, n, bad, 0), "pool check");
-    cuda_check(qm::launch_count_non_unit(stage_pert, n, bad, 0), "pool check");
-    unsigned h_bad = 0;
-    cuda_check(cudaMemcpy(&h_bad, bad, sizeof(unsigned), cudaMemcpyDeviceToHost), "pool check");
-    if (h_bad) invalid("sample-pool vectors must be unit vectors (squared length in [0.25, 4])");
+    qm::PoolStats* stats = s->d_pool_stats.as<qm::PoolStats>();
+    cuda_check(cudaMemsetAsync(stats, 0, sizeof(qm::PoolStats), 0), "pool check");
+    cuda_check(qm::launch_pool_stats(stage_dirs, stage_pert, 3, n, stats, 0), "pool check");
+    qm::PoolStats found;
+    cuda_check(cudaMemcpy(&found, stats, sizeof(found), cudaMemcpyDeviceToHost), "pool check");
+    if (found.bad) invalid("sample-pool vectors must be unit vectors (squared length in [0.25, 4])");
     cuda_check(qm::launch_xyz_to_float4(stage_dirs, s->d_samples.as<float4>(), n, 0), "pool convert");
     cuda_check(qm::launch_xyz_to_float4(stage_pert, s->d_perturb.as<float4>(), n, 0), "pool convert");
-    cuda_check(cudaDeviceSynchronize(), "pool convert");
-    rotate_pool(s, true);
+    set_pool_bounds(s, found);
+    rotate_pool(s);
   });
 }
 
@@ -1071,7 +1100,12 @@ int qmcrt_debug_shadow_free(qmcrt_scene* s, int* flags) {
   return guarded([&] {
     checked(s);
     if (!flags) invalid("output is NULL");
-    for (size_t i = 0; i < s->templates.size(); ++i) flags[i] = s->templates[i].shadow_free;
+    DeviceGuard guard(s->device);
+    std::vector<DevTask> tasks(s->templates.size());
+    if (!tasks.empty())
+      cuda_check(cudaMemcpy(tasks.data(), s->d_templates.p, tasks.size() * sizeof(DevTask), cudaMemcpyDeviceToHost),
+                 "task readback");
+    for (size_t i = 0; i < tasks.size(); ++i) flags[i] = tasks[i].shadow_free;
   });
 }
 
@@ -1195,18 +1229,16 @@ int qmcrt_debug_hit_records(qmcrt_scene* s, int id, int fb, int fe, int lb, int 
     std::vector<DevReceiver> recv = s->receivers;
     size_t maxpix = 1;
     for (auto& r : recv) maxpix = std::max(maxpix, (size_t)r.resolution.x * r.resolution.y);
-    DBuf img, dr, rec, pw, dg, task, prefix;
+    DBuf img, dr, rec, pw, dg;
     img.alloc(maxpix * sizeof(float));
     for (auto& r : recv) r.image = img.as<float>();
     upload(dr, recv);
     rec.alloc(count * sizeof(int32_t));
     pw.alloc(s->model.heliostats.size() * sizeof(double) + 8);
     dg.alloc(qm::kDiagSlots * sizeof(unsigned long long));
-    std::vector<DevTask> one{s->templates[id]};
-    upload(task, one);
     qm::TraceParams p = base_params(s);
     p.receivers = dr.as<DevReceiver>();
-    p.tasks = task.as<DevTask>();
+    p.tasks = s->d_templates.as<DevTask>() + id;
     p.num_tasks = 1;
     p.power = pw.as<double>();
     p.diag = dg.as<unsigned long long>();

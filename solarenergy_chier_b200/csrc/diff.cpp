@@ -43,6 +43,8 @@ struct qmcrt_diff {
   int radius = 0;
   std::vector<float> weights;
   DBuf d_weights, d_dtasks, d_bits, d_flux, d_tmp, d_target, d_resid, d_p, d_grad, d_loss, d_p_receivers;
+  std::vector<float4> params;  // per heliostat: aim offset, normal offset
+  DBuf d_params;
   DBuf d_deposit;  // FP64 deposit of the forward, one double per image pixel
   std::vector<qm::DevReceiver> p_receivers;
   size_t image_floats = 0;
@@ -55,7 +57,7 @@ struct qmcrt_diff {
       cudaSetDevice(batch->device);
       cudaDeviceSynchronize();
       for (DBuf* b : {&d_weights, &d_dtasks, &d_bits, &d_flux, &d_tmp, &d_target, &d_resid, &d_p, &d_grad, &d_loss,
-                      &d_p_receivers, &d_deposit})
+                      &d_p_receivers, &d_params, &d_deposit})
         b->release();
       cudaSetDevice(prev);
       qmcrt_batch_free(batch);
@@ -124,6 +126,9 @@ void diff_create(qmcrt_scene* s, const float* sun_dirs, int n_suns, float sigma_
                b->items[I.task_base + h].aim_v);
     }
   }
+  upload(b->d_items, b->items);
+  d->params.assign(d->H, make_float4(0.f, 0.f, 0.f, 0.f));
+  upload(d->d_params, d->params);
   d->radius = (int)std::ceil(3.0f * sigma_px);
   double sum = 0.0;
   std::vector<double> w(d->radius + 1);
@@ -163,6 +168,15 @@ std::vector<double> per_heliostat(const qmcrt_diff* d, const std::vector<double>
   return out;
 }
 
+// The geometry of the current parameters, prepared on the device.
+void prepare_params(qmcrt_diff* d, cudaStream_t st) {
+  if (!d->params.empty())
+    cuda_check(cudaMemcpyAsync(d->d_params.p, d->params.data(), d->params.size() * sizeof(float4),
+                               cudaMemcpyHostToDevice, st),
+               "parameter upload");
+  batch_prepare(d->batch, st, d->d_params.as<float4>());
+}
+
 void check_receiver(const qmcrt_diff* d, int receiver) {
   if (receiver < 0 || receiver >= (int)d->batch->receivers.size())
     invalid("receiver index out of range (sun k, receiver r: k x receivers + r)");
@@ -192,21 +206,15 @@ void qmcrt_diff_free(qmcrt_diff* d) { delete d; }
 int qmcrt_diff_set_params(qmcrt_diff* d, const float* aim_offsets, const float* normal_offsets) {
   return guarded([&] {
     diff_checked(d);
+    std::vector<float4> params(d->H, make_float4(0.f, 0.f, 0.f, 0.f));
     for (int h = 0; h < d->H; ++h) {
-      const float2 a = aim_offsets ? make_float2(aim_offsets[2 * h], aim_offsets[2 * h + 1]) : make_float2(0.f, 0.f);
-      const float2 n =
-          normal_offsets ? make_float2(normal_offsets[2 * h], normal_offsets[2 * h + 1]) : make_float2(0.f, 0.f);
-      if (!std::isfinite(a.x) || !std::isfinite(a.y) || !std::isfinite(n.x) || !std::isfinite(n.y))
+      float4& v = params[h];
+      if (aim_offsets) v.x = aim_offsets[2 * h], v.y = aim_offsets[2 * h + 1];
+      if (normal_offsets) v.z = normal_offsets[2 * h], v.w = normal_offsets[2 * h + 1];
+      if (!std::isfinite(v.x) || !std::isfinite(v.y) || !std::isfinite(v.z) || !std::isfinite(v.w))
         invalid("parameters must be finite");
     }
-    for (const auto& I : d->batch->inst) {
-      for (int h = 0; h < d->H; ++h) {
-        qm::PrepItem& it = d->batch->items[I.task_base + h];
-        it.aim_offset = aim_offsets ? make_float2(aim_offsets[2 * h], aim_offsets[2 * h + 1]) : make_float2(0.f, 0.f);
-        it.normal_offset =
-            normal_offsets ? make_float2(normal_offsets[2 * h], normal_offsets[2 * h + 1]) : make_float2(0.f, 0.f);
-      }
-    }
+    d->params.swap(params);
     d->forward_done = false;
   });
 }
@@ -241,13 +249,14 @@ int qmcrt_fwd(qmcrt_diff* d, double* loss, void* stream) {
     qmcrt_batch* b = d->batch;
     cudaStream_t st = static_cast<cudaStream_t>(stream);
     DeviceGuard guard(b->device);
-    batch_prepare(b, st);
-    cuda_check(qm::launch_diff_prep(b->d_items.as<qm::PrepItem>(), (int)b->items.size(), b->d_tasks.as<qm::DevTask>(),
-                                    d->d_dtasks.as<qm::DiffTask>(), st),
+    prepare_params(d, st);
+    cuda_check(qm::launch_diff_prep(prep_inputs(b, d->d_params.as<float4>()), d->d_dtasks.as<qm::DiffTask>(), st),
                "diff preparation");
     if (b->total_chunks < 0) batch_build_prefix(b);
     const size_t bits_bytes = (size_t)std::max<long long>(b->total_chunks, 1) * qm::kChunkIters * sizeof(uint32_t);
-    if (d->hit_mode == 0) {
+    if (d->hit_mode == 0 && bits_bytes <= d->d_bits.bytes) {
+      d->recompute = false;  // the checkpoint is there already
+    } else if (d->hit_mode == 0) {
       size_t free_b = 0, total_b = 0;
       cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
       d->recompute = bits_bytes > d->d_bits.bytes + free_b / 4;
@@ -370,7 +379,7 @@ int qmcrt_diff_plain(qmcrt_diff* d, void* stream) {
     // The same parameterised geometry and rays as the forward, binned to
     // the nearest pixel as the plain tracer does.  The forward's hit bits,
     // residual and tangents are untouched, so a pending qmcrt_bwd stays valid.
-    batch_prepare(b, st);
+    prepare_params(d, st);
     if (b->total_chunks < 0) batch_build_prefix(b);
     cuda_check(cudaMemsetAsync(b->d_images.p, 0, b->d_images.bytes, st), "clear");
     cuda_check(cudaMemsetAsync(b->d_power.p, 0, b->d_power.bytes, st), "clear");

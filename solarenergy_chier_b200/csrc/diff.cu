@@ -184,15 +184,17 @@ __device__ __forceinline__ Dual3T<N> to_world(const DFrameT<N>& f, float3 d) {
 }
 
 // ---- preparation: normal and frame of every heliostat with tangents --------
-__global__ void diff_prep_kernel(const PrepItem* items, int n, const DevTask* tasks, DiffTask* out) {
+__global__ void diff_prep_kernel(PrepInputs p, DiffTask* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const PrepItem it = items[i];
-  const DevTask& T = tasks[it.task];
+  if (i >= p.n) return;
+  const PrepItem it = p.items[i];
+  const DevTask& T = p.tasks[it.task];
+  const float3 sun_dir = p.suns[it.sun].dir;
+  const float4 offset = p.params[it.param];
   // aim point a = focus + du aim_u + dv aim_v
-  Dual3T<K> a = d3<K>(make_float3(it.focus.x + it.aim_u.x * it.aim_offset.x + it.aim_v.x * it.aim_offset.y,
-                           it.focus.y + it.aim_u.y * it.aim_offset.x + it.aim_v.y * it.aim_offset.y,
-                           it.focus.z + it.aim_u.z * it.aim_offset.x + it.aim_v.z * it.aim_offset.y));
+  Dual3T<K> a = d3<K>(make_float3(it.focus.x + it.aim_u.x * offset.x + it.aim_v.x * offset.y,
+                                  it.focus.y + it.aim_u.y * offset.x + it.aim_v.y * offset.y,
+                                  it.focus.z + it.aim_u.z * offset.x + it.aim_v.z * offset.y));
   a.x.d[0] = it.aim_u.x;
   a.y.d[0] = it.aim_u.y;
   a.z.d[0] = it.aim_u.z;
@@ -200,10 +202,10 @@ __global__ void diff_prep_kernel(const PrepItem* items, int n, const DevTask* ta
   a.y.d[1] = it.aim_v.y;
   a.z.d[1] = it.aim_v.z;
   const Dual3T<K> r = normalize(a - d3<K>(T.pos));
-  const Dual3T<K> n0 = normalize(r - d3<K>(it.sun_dir));
+  const Dual3T<K> n0 = normalize(r - d3<K>(sun_dir));
   const DFrameT<K> f0 = make_dframe(n0, false);
   const Dual3T<K> nrm =
-      normalize(n0 + f0.u * dvar<K>(it.normal_offset.x, 2) + f0.v * dvar<K>(it.normal_offset.y, 3));
+      normalize(n0 + f0.u * dvar<K>(offset.z, 2) + f0.v * dvar<K>(offset.w, 3));
   const DFrameT<K> hf = make_dframe(nrm, T.type == 1);
   DiffTask o;
   o.n = nrm;
@@ -354,7 +356,7 @@ __device__ __forceinline__ void ray_adjoint(const ChunkConstants& T, const Facet
     rr = x * x + z * z;
     dxz2 = d.x * d.x + d.z * d.z;
     if (!(rr > 0.0f) || !(dxz2 > 0.0f)) return;
-    band = !(den * den > kGrazing * kGrazing * (rr * dxz2));
+    band = !(fabsf(den) > kGrazing * sqrtf(rr * dxz2));  // rounded thus: one ray on the other side shows
   }
   if (band) {
     // Silhouette band: rays whose impact parameter b (distance of the
@@ -648,9 +650,10 @@ __global__ void loss_kernel(const float* flux, const float* target, float* resid
 
 }  // namespace
 
-cudaError_t launch_diff_prep(const PrepItem* items, int n, const DevTask* tasks, DiffTask* out, cudaStream_t stream) {
-  if (n <= 0) return cudaSuccess;
-  diff_prep_kernel<<<(n + 127) / 128, 128, 0, stream>>>(items, n, tasks, out);
+cudaError_t launch_diff_prep(const PrepInputs& p, DiffTask* out, cudaStream_t stream) {
+  if (p.n <= 0) return cudaSuccess;
+  if (!p.params) return cudaErrorInvalidValue;
+  diff_prep_kernel<<<(p.n + 31) / 32, 32, 0, stream>>>(p, out);
   return cudaGetLastError();
 }
 

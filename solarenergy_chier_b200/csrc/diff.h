@@ -46,7 +46,7 @@ struct BackwardParams {
   double* grad;                   // kDiffParams per power slot
 };
 
-cudaError_t launch_diff_prep(const PrepItem* items, int n, const DevTask* tasks, DiffTask* out, cudaStream_t stream);
+cudaError_t launch_diff_prep(const PrepInputs& p, DiffTask* out, cudaStream_t stream);
 cudaError_t launch_diff_backward(const BackwardParams& p, cudaStream_t stream);
 
 // Separable normalised Gaussian of `radius` taps each side (weights[0..radius])

@@ -119,31 +119,28 @@ __global__ void trace_pools_kernel(const float4* in, const float4* pert, int n, 
   out[i] = make_float4(d.x, d.y, d.z, 0.0f);
 }
 
-// Largest tan(angle from +y) of a pool, as float bits (non-negative floats
-// order like their bit patterns); +inf when some direction has y <= 0.
-__global__ void pool_tan_kernel(const float4* pool, int n, unsigned* out) {
+// Both pools' checks and bounds in one pass: vectors whose squared length
+// lies outside [0.25, 4] or is NaN, and the largest tan(angle from +y) of each
+// pool as float bits (non-negative floats order like their bit patterns); +inf
+// when some direction has y <= 0.
+__global__ void pool_stats_kernel(const float* dirs, const float* perts, int stride, int n, PoolStats* out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  float t = 0.0f;
-  if (i < n) {
-    const float4 q = pool[i];
-    t = q.y > 0.0f ? sqrtf(q.x * q.x + q.z * q.z) / q.y : __int_as_float(0x7f800000);
+  unsigned bad = 0;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    float t = 0.0f;
+    if (i < n) {
+      const float* v = (k ? perts : dirs) + (size_t)stride * i;
+      const float x = v[0], y = v[1], z = v[2];
+      const float s = x * x + y * y + z * z;
+      bad += !(s >= 0.25f && s <= 4.0f);
+      t = y > 0.0f ? sqrtf(x * x + z * z) / y : __int_as_float(0x7f800000);
+    }
+    const unsigned most = __reduce_max_sync(0xffffffffu, __float_as_uint(t));
+    if ((threadIdx.x & 31) == 0) atomicMax(out->tan_bits + k, most);
   }
-  for (int off = 16; off > 0; off >>= 1) t = fmaxf(t, __shfl_down_sync(0xffffffffu, t, off));
-  if ((threadIdx.x & 31) == 0) atomicMax(out, __float_as_uint(t));
-}
-
-// Counts the xyz vectors whose squared length lies outside [0.25, 4] or is
-// NaN (one warp-aggregated atomic per warp).
-__global__ void count_non_unit_kernel(const float* xyz, int n, unsigned* bad) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  bool b = false;
-  if (i < n) {
-    const float x = xyz[3 * i], y = xyz[3 * i + 1], z = xyz[3 * i + 2];
-    const float s = x * x + y * y + z * z;
-    b = !(s >= 0.25f && s <= 4.0f);
-  }
-  const unsigned votes = __ballot_sync(0xffffffffu, b);
-  if ((threadIdx.x & 31) == 0 && votes) atomicAdd(bad, (unsigned)__popc(votes));
+  bad = __reduce_add_sync(0xffffffffu, bad);
+  if ((threadIdx.x & 31) == 0 && bad) atomicAdd(&out->bad, bad);
 }
 
 __global__ void xyz_to_float4_kernel(const float* xyz, float4* out, int n) {
@@ -180,15 +177,10 @@ cudaError_t launch_trace_pools(const float4* samples, const float4* perturbation
   return cudaGetLastError();
 }
 
-cudaError_t launch_pool_tan(const float4* pool, int n, unsigned* out, cudaStream_t stream) {
+cudaError_t launch_pool_stats(const float* dirs, const float* perts, int stride, int n, PoolStats* out,
+                              cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
-  pool_tan_kernel<<<(n + 255) / 256, 256, 0, stream>>>(pool, n, out);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_count_non_unit(const float* xyz, int n, unsigned* bad, cudaStream_t stream) {
-  if (n <= 0) return cudaSuccess;
-  count_non_unit_kernel<<<(n + 255) / 256, 256, 0, stream>>>(xyz, n, bad);
+  pool_stats_kernel<<<(n + 255) / 256, 256, 0, stream>>>(dirs, perts, stride, n, out);
   return cudaGetLastError();
 }
 

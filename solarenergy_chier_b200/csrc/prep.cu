@@ -19,19 +19,24 @@
 namespace qm {
 namespace {
 
-__global__ void prep_kernel(const PrepItem* items, int n, DevTask* tasks) {
+// A thread per heliostat, in blocks of one warp so that a few hundred
+// heliostats still spread over the SMs: a chain of dependent double
+// arithmetic per sub-heliostat, 16 us for 648 heliostats of 4, 86 us for 1,872
+// of 28.  Moving a plain scene's sun here from the host (with its uploads)
+// took a sun of 648 heliostats from 1.6 to 0.5 ms, its trace included.
+__global__ void prep_kernel(PrepInputs p) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const PrepItem it = items[i];
-  DevTask& T = tasks[it.task];
+  if (i >= p.n) return;
+  const PrepItem it = p.items[i];
+  DevTask& T = p.tasks[it.task];
+  const float4 offset = p.params ? p.params[it.param] : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
   float3 aim = it.focus;
-  if (it.aim_offset.x != 0.0f || it.aim_offset.y != 0.0f)
-    aim = qs::add(qs::add(aim, qs::mul(it.aim_u, it.aim_offset.x)), qs::mul(it.aim_v, it.aim_offset.y));
-  float3 normal = helio_normal(T.pos, aim, it.sun_dir);
-  if (it.normal_offset.x != 0.0f || it.normal_offset.y != 0.0f) {
+  if (offset.x != 0.0f || offset.y != 0.0f)
+    aim = qs::add(qs::add(aim, qs::mul(it.aim_u, offset.x)), qs::mul(it.aim_v, offset.y));
+  float3 normal = helio_normal(T.pos, aim, p.suns[it.sun].dir);
+  if (offset.z != 0.0f || offset.w != 0.0f) {
     const Frame f0 = qs::make_frame(normal, false);
-    normal = qs::normalize(
-        qs::add(qs::add(normal, qs::mul(f0.u, it.normal_offset.x)), qs::mul(f0.v, it.normal_offset.y)));
+    normal = qs::normalize(qs::add(qs::add(normal, qs::mul(f0.u, offset.z)), qs::mul(f0.v, offset.w)));
   }
   T.normal = normal;
   const Frame hf = qs::make_frame(normal, T.type == 1);
@@ -92,18 +97,19 @@ __device__ __forceinline__ float3 sub_normal(const DevTask& T, int s) {
 // Walk codes of the prepared tasks: warp j handles task j / (1 + max_sub),
 // slot j % (1 + max_sub): slot 0 its shadow walks, slot 1 + s the block
 // walks of its sub-heliostat s (each a capsule enumeration of its own).
-__global__ void shadow_kernel(const PrepItem* items, int n, int max_sub, DevTask* tasks, const DevGrid* grids) {
+__global__ void shadow_kernel(PrepInputs p, int max_sub, const DevGrid* grids) {
   const long long j = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int lane = threadIdx.x & 31;
   const int i = (int)(j / (1 + max_sub)), slot = (int)(j % (1 + max_sub));
-  if (i >= n) return;
-  const PrepItem& it = items[i];
-  DevTask& T = tasks[it.task];
+  if (i >= p.n) return;
+  const PrepItem& it = p.items[i];
+  const SunParams& sun = p.suns[it.sun];
+  DevTask& T = p.tasks[it.task];
   const DevGrid& G = grids[T.grid];
   const ShadowGrid view{G.pos, G.interval, G.cells, G.bound, G.cell_range, G.entries};
   Cone cone;
   if (slot == 0) {
-    const int state = it.shadow_tan >= 0.0f ? shadow_cone(view, T.own, it.shadow_axis, it.shadow_tan, cone) : -1;
+    const int state = sun.shadow_tan >= 0.0f ? shadow_cone(view, T.own, sun.shadow_axis, sun.shadow_tan, cone) : -1;
     const int code = warp_code(view, T.own, state, cone, T.shadow_cand);
     if (lane == 0) T.shadow_free = code;
     return;
@@ -111,44 +117,19 @@ __global__ void shadow_kernel(const PrepItem* items, int n, int max_sub, DevTask
   const int s = slot - 1;
   if (s >= it.num_sub) return;
   if (lane == 0) sub_frames(T, s, it.sub_frames + 6 * s);
-  const int state = it.block_theta >= 0.0f
-                        ? block_cone(view, it.verts + 3 * s, it.sun_dir, sub_normal(T, s), it.block_theta, cone)
+  const int state = sun.block_theta >= 0.0f
+                        ? block_cone(view, it.verts + 3 * s, sun.dir, sub_normal(T, s), sun.block_theta, cone)
                         : -1;
   const int code = warp_code(view, T.own, state, cone, it.sub_cand + kMaxCandidates * s);
   if (lane == 0) it.sub_free[s] = code;
 }
 
-// Walk codes of a plain scene's heliostats (its task templates), with the
-// same warp layout as shadow_kernel; the sub-heliostat parallelograms are
-// read back from the traversal form (A, B - A, C - A) -- the tests are
-// conservative far above that rounding.
-__global__ void walk_flags_kernel(WalkFlagParams p) {
-  const long long j = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int i = (int)(j / (1 + p.max_sub)), slot = (int)(j % (1 + p.max_sub));
-  if (i >= p.n) return;
-  const DevTask& T = p.tasks[i];
-  const DevGrid& G = p.grids[T.grid];
-  const ShadowGrid view{G.pos, G.interval, G.cells, G.bound, G.cell_range, G.entries};
-  Cone cone;
-  if (slot == 0) {
-    const int state = p.sun_tan >= 0.0f ? shadow_cone(view, T.own, p.sun_axis, p.sun_tan, cone) : -1;
-    const int code = warp_code(view, T.own, state, cone, p.shadow_cand_out + kMaxCandidates * i);
-    if (lane == 0) p.shadow_out[i] = code;
-    return;
-  }
-  const int s = slot - 1;
-  const int4 hs = G.hsub[T.own];
-  if (s >= hs.y) return;
-  if (lane == 0) sub_frames(T, s, const_cast<float4*>(G.sub_frames) + 6 * (hs.x + s));
-  const float4* q = G.subv + 3 * (hs.x + s);
-  const float3 A = make_float3(q[0].x, q[0].y, q[0].z);
-  const float3 bac[3] = {make_float3(A.x + q[0].w, A.y + q[1].x, A.z + q[1].y), A,
-                         make_float3(A.x + q[1].z, A.y + q[1].w, A.z + q[2].x)};
-  const int state =
-      p.block_theta >= 0.0f ? block_cone(view, bac, p.sun_dir, sub_normal(T, s), p.block_theta, cone) : -1;
-  const int code = warp_code(view, T.own, state, cone, const_cast<int*>(G.sub_cand) + kMaxCandidates * (hs.x + s));
-  if (lane == 0) const_cast<int*>(G.sub_free)[hs.x + s] = code;
+__global__ void gather_tasks_kernel(const DevTask* tasks, const int* ids, int n, DevTask* out) {
+  constexpr int kWords = sizeof(DevTask) / 4;
+  static_assert(sizeof(DevTask) % 4 == 0, "copied by words");
+  const long long j = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = (int)(j / kWords), w = (int)(j % kWords);
+  if (i < n) reinterpret_cast<int*>(out + i)[w] = reinterpret_cast<const int*>(tasks + ids[i])[w];
 }
 
 // Pool of instance blockIdx.y turned by that instance's sun frame.
@@ -171,30 +152,26 @@ __global__ void rotate_pools_kernel(const PoolRotation* jobs) {
 
 }  // namespace
 
-cudaError_t launch_prep(const PrepItem* items, int n, DevTask* tasks, cudaStream_t stream) {
-  if (n <= 0) return cudaSuccess;
-  prep_kernel<<<(n + 127) / 128, 128, 0, stream>>>(items, n, tasks);
+cudaError_t launch_prep(const PrepInputs& p, cudaStream_t stream) {
+  if (p.n <= 0) return cudaSuccess;
+  prep_kernel<<<(p.n + 31) / 32, 32, 0, stream>>>(p);
   return cudaGetLastError();
 }
 
-cudaError_t launch_shadow_flags(const PrepItem* items, int n, int max_sub, DevTask* tasks, const DevGrid* grids,
-                                cudaStream_t stream) {
-  if (n <= 0) return cudaSuccess;
+cudaError_t launch_shadow_flags(const PrepInputs& p, int max_sub, const DevGrid* grids, cudaStream_t stream) {
+  if (p.n <= 0) return cudaSuccess;
   if (max_sub < 0) return cudaErrorInvalidValue;
-  const long long warps = (long long)n * (1 + max_sub);
+  const long long warps = (long long)p.n * (1 + max_sub);
   const long long blocks = (warps + 3) / 4;  // four warps a block, a warp per cone
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-  shadow_kernel<<<(unsigned)blocks, 128, 0, stream>>>(items, n, max_sub, tasks, grids);
+  shadow_kernel<<<(unsigned)blocks, 128, 0, stream>>>(p, max_sub, grids);
   return cudaGetLastError();
 }
 
-cudaError_t launch_walk_flags(const WalkFlagParams& p, cudaStream_t stream) {
-  if (p.n <= 0) return cudaSuccess;
-  if (p.max_sub < 0) return cudaErrorInvalidValue;
-  const long long warps = (long long)p.n * (1 + p.max_sub);
-  const long long blocks = (warps + 3) / 4;
-  if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
-  walk_flags_kernel<<<(unsigned)blocks, 128, 0, stream>>>(p);
+cudaError_t launch_gather_tasks(const DevTask* tasks, const int* ids, int n, DevTask* out, cudaStream_t stream) {
+  if (n <= 0) return cudaSuccess;
+  const long long words = (long long)n * (sizeof(DevTask) / 4);
+  gather_tasks_kernel<<<(unsigned)((words + 255) / 256), 256, 0, stream>>>(tasks, ids, n, out);
   return cudaGetLastError();
 }
 

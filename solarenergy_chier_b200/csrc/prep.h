@@ -7,28 +7,30 @@
 
 namespace qm {
 
-// One (sun, heliostat) to prepare.  The task already holds the heliostat's
-// sun-independent fields; the kernel fills its normal and facet frame and
-// writes the heliostat's sub-heliostat parallelograms and traversal record
-// into the sun's grid arrays.
+// One sun of a preparation: its direction of travel, and what the walk-free
+// tests need (csrc/shadow.h): the axis toward the sun with the world-space
+// tangent of the largest sun-shape angle (< 0: unbounded, no test), and
+// theta_sun + 2 theta_slope (< 0: no test).
+struct SunParams {
+  float3 dir;
+  float3 shadow_axis;
+  float shadow_tan;
+  float block_theta;
+};
+
+// One (sun, heliostat) to prepare, the same for every sun direction: uploaded
+// once, so that a new sun costs its SunParams alone.  The task already holds
+// the heliostat's sun-independent fields; the kernels fill its normal, facet
+// frame and walk code and write the heliostat's sub-heliostat parallelograms
+// and traversal record into the sun's grid arrays.
 struct PrepItem {
   int task;         // index into the task array
+  int sun;          // index into the SunParams
+  int param;        // index into the differentiable parameters
   int num_sub;      // sub-heliostats of the heliostat
   int sub_first;    // grid-local id of its first sub-heliostat
   float3 focus;     // aim point (sun-independent)
-  float3 sun_dir;   // direction of travel of the sun's rays
-  // Differentiable parameters (zero for plain batches): the aim point moves
-  // by aim_offset.x * aim_u + aim_offset.y * aim_v; the normal then turns by
-  // normal_offset (radians) about the u and v axes of its own frame.
-  float2 aim_offset, normal_offset;
-  float3 aim_u, aim_v;
-  // Shadow-free test (qm::shadow_free): sun axis and world-space tangent of
-  // the largest sun-shape angle (< 0: unbounded, never shadow-free).
-  float3 shadow_axis;
-  float shadow_tan;
-  // Block-free test (qm::block_free): theta_sun + 2 theta_slope (< 0: never),
-  // and where the heliostat's per-sub-heliostat flags go.
-  float block_theta;
+  float3 aim_u, aim_v;  // aim axes of the differentiable parameters
   int* sub_free;
   int* sub_cand;  // kMaxCandidates per sub-heliostat
   float4* sub_frames;  // 6 per sub-heliostat (DevGrid::sub_frames)
@@ -38,6 +40,18 @@ struct PrepItem {
   int4* hsub;       // out: (first, count, lattice rows, lattice columns)
 };
 
+// Inputs of the preparation kernels.  params (NULL: none): per heliostat
+// (aim x, aim y, normal x, normal y): the aim point moves by x aim_u + y
+// aim_v; the normal then turns by (x, y) radians about the u and v axes of its
+// own frame.
+struct PrepInputs {
+  const PrepItem* items;
+  int n;
+  DevTask* tasks;
+  const SunParams* suns;
+  const float4* params;
+};
+
 struct PoolRotation {
   const float4* in;  // local sun-shape pool, n entries
   float4* out;       // world-space tracer copy, n_out = n + L entries (entry i = pool entry i % n)
@@ -45,29 +59,14 @@ struct PoolRotation {
   SunFrame sun;
 };
 
-// Walk-free flags of a plain scene: shadow flags per task into shadow_out,
-// block flags per sub-heliostat into each grid's sub_free array.
-struct WalkFlagParams {
-  const DevTask* tasks;
-  int n;
-  const DevGrid* grids;
-  float3 sun_axis;  // toward the sun
-  float sun_tan;    // tan of the largest sun-shape angle (< 0: unbounded)
-  float3 sun_dir;   // direction of travel
-  float block_theta;
-  int* shadow_out;       // per task: DevTask::shadow_free code
-  int* shadow_cand_out;  // per task: kMaxCandidates DevTask::shadow_cand entries
-  int max_sub;           // most sub-heliostats of any task
-};
-cudaError_t launch_walk_flags(const WalkFlagParams& p, cudaStream_t stream);
-
-cudaError_t launch_prep(const PrepItem* items, int n, DevTask* tasks, cudaStream_t stream);
-// Shadow-free flags of the prepared tasks; grids: the tasks' grids with their
-// prepared traversal records.  Run after launch_prep.
+cudaError_t launch_prep(const PrepInputs& p, cudaStream_t stream);
+// Walk codes and sub-heliostat frames of the prepared tasks; grids: the
+// tasks' grids with their prepared traversal records.  Run after launch_prep.
 // max_sub: the most sub-heliostats of any item (one warp per heliostat and
 // per sub-heliostat).
-cudaError_t launch_shadow_flags(const PrepItem* items, int n, int max_sub, DevTask* tasks, const DevGrid* grids,
-                                cudaStream_t stream);
+cudaError_t launch_shadow_flags(const PrepInputs& p, int max_sub, const DevGrid* grids, cudaStream_t stream);
+// out[i] = tasks[ids[i]].
+cudaError_t launch_gather_tasks(const DevTask* tasks, const int* ids, int n, DevTask* out, cudaStream_t stream);
 // max_out: the largest n_out of the jobs.
 cudaError_t launch_rotate_pools(const PoolRotation* jobs, int n_jobs, int max_out, cudaStream_t stream);
 

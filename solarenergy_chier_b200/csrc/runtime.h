@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "device_scene.h"
+#include "prep.h"
 #include "qmcrt.h"
 #include "scene.h"
 
@@ -95,7 +96,7 @@ void upload(DBuf& b, const std::vector<T>& v) {
 }
 
 struct GridBufs {
-  DBuf ranges, entries, bound, hsub, subv, sub_free, sub_cand, sub_frames;
+  DBuf ranges, entries, bound, hsub, subv, verts, sub_free, sub_cand, sub_frames;
 };
 
 class DeviceGuard {
@@ -137,7 +138,7 @@ struct qmcrt_scene {
   bool flags_valid = false;
   float3 flags_sun{};
   float flags_tan = 0.f, flags_slope = 0.f;
-  qrt::DBuf d_flag_tasks, d_flag_out, d_scratch_word;
+  qrt::DBuf d_pool_stats;  // results of the pool checks
   qrt::DBuf d_pool_stage;  // staging of qmcrt_set_sample_pool uploads
   qrt::DBuf d_trace_samples;  // tracer copy: d_samples in world space, P + L entries (entry i = i % P)
   qrt::DBuf d_trace_perturb;  // tracer copy of d_perturb, P + L entries
@@ -146,14 +147,23 @@ struct qmcrt_scene {
   qrt::DBuf d_power, d_diag;
   qrt::DBuf d_chunk_power;  // per-chunk FP64 power partials of a launch (grows to the largest launch)
   qrt::DBuf d_work;         // work counter of persistent flux launches
+  // One task per heliostat.  The host copy holds what does not depend on the
+  // sun; the normals, frames and walk codes are the device copy's alone,
+  // prepared there for every new sun from d_items and d_sun.
   std::vector<qm::DevTask> templates;
-  qrt::DBuf d_tasks, d_prefix;
+  qrt::DBuf d_templates, d_items, d_sun;
+  int max_sub = 0;                 // most sub-heliostats of any heliostat
+  mutable bool model_stale = false;  // the model's normals and vertices are an earlier sun's
+  // Traced lists: consecutive heliostats are traced from d_templates itself,
+  // others from a copy in list order (d_tasks, of the sun it was gathered for).
+  qrt::DBuf d_tasks, d_ids, d_prefix, d_single;
   std::vector<int> cached_ids;
   long long cached_lights = -1;
   long long cached_chunk = -1;
+  bool gathered = false;
+  long long single_lights = -1, single_chunk = -1;  // d_single: chunks of each heliostat traced alone
   int shape = 0;  // launch shape of the production build (qmcrt_set_launch_shape)
-  bool cache_valid = false;
-  qm::DevTask* h_stage = nullptr;  // pinned staging for task uploads
+  int* h_ids = nullptr;  // pinned staging of list uploads
   long long* h_prefix = nullptr;
   size_t stage_cap = 0;
   cudaEvent_t stage_done = nullptr;
@@ -168,7 +178,7 @@ struct qmcrt_scene {
     cudaGetDevice(&prev);
     cudaSetDevice(device);
     cudaDeviceSynchronize();
-    if (h_stage) cudaFreeHost(h_stage);
+    if (h_ids) cudaFreeHost(h_ids);
     if (h_prefix) cudaFreeHost(h_prefix);
     if (stage_done) cudaEventDestroy(stage_done);
     grid_bufs.clear();
@@ -180,9 +190,12 @@ struct qmcrt_scene {
     d_samples.release();
     d_perturb.release();
     d_trace_samples.release();
-    d_flag_tasks.release();
-    d_flag_out.release();
-    d_scratch_word.release();
+    d_pool_stats.release();
+    d_templates.release();
+    d_items.release();
+    d_sun.release();
+    d_ids.release();
+    d_single.release();
     d_pool_stage.release();
     d_trace_perturb.release();
     d_offset_seg.release();
@@ -200,12 +213,13 @@ struct qmcrt_scene {
 namespace qrt {
 
 // Scene helpers defined in capi.cpp.
-void grid_sun_data(const qm::SceneModel& m, const qm::GridModel& g, std::vector<float4>& bound,
-                   std::vector<int4>& hsub, std::vector<float4>& subv);
 qmcrt_scene* checked(qmcrt_scene* s);
-// Sun axis and world-space tangent of the largest sun-shape angle for the
-// shadow-free test (tan_local < 0: unbounded, tan_world < 0).
-void sun_cone(float3 sun_dir, float tan_local, float3& axis, float& tan_world);
+// Frame of the reversed sun direction, which turns the sun-shape pool into
+// world space.
+qm::SunFrame sun_frame(float3 sun_dir);
+// A sun's preparation parameters from the pools' bounds (tan_local,
+// slope_angle < 0: unbounded, no walk-free tests).
+qm::SunParams sun_params(float3 sun_dir, float tan_local, float slope_angle);
 // out: 0 flux, 1 per-ray outcome codes, 2 bilinear deposit, 3 hit bits
 // (qm::TraceOut in tracer.cu); mode: the kernel build (qmcrt_set_math_mode);
 // work_counter: one device word, used by flux launches of the persistent shape.
