@@ -59,7 +59,7 @@ void batch_prepare(qmcrt_batch* b, cudaStream_t st, const float4* params) {
   cuda_check(cudaMemcpyAsync(b->d_suns.p, suns.data(), suns.size() * sizeof(qm::SunParams), cudaMemcpyHostToDevice, st),
              "sun upload");
   const qm::PrepInputs in = prep_inputs(b, params);
-  cuda_check(qm::launch_prep(in, st), "prep kernel");
+  cuda_check(qm::launch_prep(in, b->d_grids.as<qm::DevGrid>(), (int)b->grids.size(), st), "prep kernel");
   cuda_check(qm::launch_shadow_flags(in, b->max_sub, b->d_grids.as<qm::DevGrid>(), st), "shadow flags");
   std::vector<qm::PoolRotation> rot(b->inst.size());
   int max_out = 0;
@@ -255,6 +255,8 @@ int qmcrt_batch_create(qmcrt_scene* const* scenes, int n_scenes, const int* scen
       it.hsub = b->d_hsub.as<int4>() + gs.hsub + item_slot[i].local;
     }
     upload(b->d_grids, b->grids);
+    for (size_t i = 0; i < b->items.size(); ++i)
+      b->items[i].top_key = &b->d_grids.as<qm::DevGrid>()[item_slot[i].grid].top_key;
     upload(b->d_receivers, b->receivers);
     upload(b->d_tasks, b->tasks);
     upload(b->d_items, b->items);

@@ -125,6 +125,7 @@ void build_templates(qmcrt_scene* s) {
     const int own = (int)i - m.grids[h.grid].start_heliostat;
     it.bound = gb.bound.as<float4>() + 5 * (size_t)own;
     it.hsub = gb.hsub.as<int4>() + own;
+    it.top_key = &s->d_grids.as<DevGrid>()[h.grid].top_key;
     s->max_sub = std::max(s->max_sub, h.num_sub);
   }
   upload(s->d_items, items);
@@ -148,7 +149,7 @@ qm::PrepInputs sun_inputs(qmcrt_scene* s) {
 
 void prepare_sun(qmcrt_scene* s) {
   s->sun = sun_frame(s->model.config.sun_dir);
-  cuda_check(qm::launch_prep(sun_inputs(s), 0), "prep kernel");
+  cuda_check(qm::launch_prep(sun_inputs(s), s->d_grids.as<DevGrid>(), (int)s->grids.size(), 0), "prep kernel");
   s->gathered = false;
 }
 
@@ -201,6 +202,7 @@ void build_device_scene(qmcrt_scene* s) {
     dg.interval = g.interval;
     dg.cells = g.cells;
     dg.max_steps = g.cells.x + g.cells.y + g.cells.z + 2;
+    dg.top_key = qm::kNoHeight;
     dg.cell_range = gb->ranges.as<int2>();
     dg.entries = gb->entries.as<int4>();
     dg.bound = gb->bound.as<float4>();

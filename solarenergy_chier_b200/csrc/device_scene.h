@@ -18,6 +18,7 @@ struct DevGrid {
   float3 interval;
   int3 cells;
   int max_steps;        // DDA step bound: cells.x + cells.y + cells.z + 2
+  int top_key;          // highest point of the padded boxes (height_key), written with the traversal records
   const int2* cell_range;  // [begin, end) of each cell's entries
   const int4* entries;     // per cell entry: grid-local heliostat id, first sub-heliostat, count, 0
   const float4* bound;  // 5 float4 per grid-local heliostat: (centre, window margin), (axis_k, half extent_k)
@@ -36,6 +37,11 @@ struct DevGrid {
   // (same layout): 6 float4, written with the walk codes for the current sun.
   const float4* sub_frames;
 };
+
+// Floats as integers of the same order, so that an integer atomic maximum
+// finds the largest (kNoHeight: below all of them, and all bytes alike).
+constexpr int kNoHeight = (int)0x80808080;
+__host__ __device__ __forceinline__ int height_key(int bits) { return bits ^ ((bits >> 31) & 0x7fffffff); }
 
 struct DevReceiver {
   int type;             // 0 rectangle, 1 cylinder

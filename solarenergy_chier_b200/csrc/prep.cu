@@ -66,6 +66,9 @@ __global__ void prep_kernel(PrepInputs p) {
   int2 rc;
   heliostat_record(v, it.num_sub, T.row_col, T.pos, normal, it.bound, &rc);
   *it.hsub = make_int4(it.sub_first, it.num_sub, rc.x, rc.y);
+  const float4 *c = it.bound;
+  atomicMax(it.top_key, height_key(__float_as_int(c[0].y + fabsf(c[1].y) * c[1].w + fabsf(c[2].y) * c[2].w +
+                                                  fabsf(c[3].y) * c[3].w)));
 }
 
 // DevGrid::sub_free code of a block_candidates result: 1 nothing to hit,
@@ -152,8 +155,11 @@ __global__ void rotate_pools_kernel(const PoolRotation* jobs) {
 
 }  // namespace
 
-cudaError_t launch_prep(const PrepInputs& p, cudaStream_t stream) {
+cudaError_t launch_prep(const PrepInputs& p, DevGrid* grids, int num_grids, cudaStream_t stream) {
   if (p.n <= 0) return cudaSuccess;
+  static_assert(kNoHeight == (int)0x80808080, "set by bytes");
+  const cudaError_t e = cudaMemset2DAsync(&grids->top_key, sizeof(DevGrid), 0x80, sizeof(int), num_grids, stream);
+  if (e != cudaSuccess) return e;
   prep_kernel<<<(p.n + 31) / 32, 32, 0, stream>>>(p);
   return cudaGetLastError();
 }

@@ -38,6 +38,7 @@ struct PrepItem {
   float4* subv;     // out: 3 float4 per sub-heliostat (A, B - A, C - A)
   float4* bound;    // out: 5 float4 traversal record
   int4* hsub;       // out: (first, count, lattice rows, lattice columns)
+  int* top_key;     // out: raised to the box's highest point (DevGrid::top_key)
 };
 
 // Inputs of the preparation kernels.  params (NULL: none): per heliostat
@@ -59,7 +60,8 @@ struct PoolRotation {
   SunFrame sun;
 };
 
-cudaError_t launch_prep(const PrepInputs& p, cudaStream_t stream);
+// grids, num_grids: the grids that the items' records belong to.
+cudaError_t launch_prep(const PrepInputs& p, DevGrid* grids, int num_grids, cudaStream_t stream);
 // Walk codes and sub-heliostat frames of the prepared tasks; grids: the
 // tasks' grids with their prepared traversal records.  Run after launch_prep.
 // max_sub: the most sub-heliostats of any item (one warp per heliostat and

@@ -305,6 +305,16 @@ __device__ __forceinline__ bool collide(const DevGrid& g, int own, float3 o, flo
   td.x = abs_divide(g.interval.x, d.x);
   td.y = abs_divide(g.interval.y, d.y);
   td.z = abs_divide(g.interval.z, d.z);
+  // A rising ray can hit nothing above the highest padded box, so in the top
+  // layer of cells the walk leaves the grid at that height (plus 5 cm, far
+  // above the rounding of heights and boundary distances and the 1e-5 ties).
+  // The reference walks on to the grid's own top; reflected rays of far
+  // heliostats rise so little that most of their cells lay above every mirror
+  // (10,000 heliostats, 256 M rays at 36 to 59 degrees of sun: 19.6 -> 12.5 ms).
+  if (d.y > 0.0f && c.y == g.cells.y - 1) {
+    const float top = __int_as_float(height_key(g.top_key));
+    tm.y = fminf(tm.y, fmaxf(__fdividef(top + (0.05f + 1e-5f * fabsf(top)) - o.y, d.y), 0.0f));
+  }
   int seen0 = -1, seen1 = -1;
   for (int it = 0; it < g.max_steps; ++it) {
     if ((unsigned)c.x >= (unsigned)g.cells.x || (unsigned)c.y >= (unsigned)g.cells.y ||

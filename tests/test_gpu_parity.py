@@ -375,6 +375,41 @@ def test_shadow_skip_keeps_per_ray_outcomes(tmp_path, sun):
     assert set(np.unique(bfree)) <= set(range(0, 8))
 
 
+@pytest.mark.parametrize("elevation", [12.0, 36.0])
+def test_walks_that_end_above_the_mirrors(elevation, tmp_path):
+    """A dense field whose far heliostats have too many possible blockers for
+    a list, so that their rays walk, and rising rays leave the walk above the
+    highest mirror: per-ray outcomes of the exact build identical to the
+    oracle's, which walks to the grid's top; the production build's decisions
+    agree on 99.99 % of the rays (one ray per heliostat sample allowed)."""
+    import json
+    from pathlib import Path
+
+    f = synth.huge_field(tmp_path, seed=5, helio_pixel=1.0, receiver_pixel=0.2, groups=4, per_group=128)
+    cfg = json.loads(Path(f.config).read_text())
+    Path(f.config).write_text(json.dumps(dict(cfg, sun_dir=synth.sun_direction(150.0, elevation))))
+    s = q.Scene(f.scene, f.config, device=0, seed=3)
+    s.generate_sample_pool(7)
+    dirs, pert = s.get_sample_pool()
+    codes = s.block_free(0)
+    walkers = np.nonzero(codes == 0)[0]
+    assert len(walkers) > 100, "no walks in this field"
+    o = oracle.OracleScene.from_files(f.scene, f.config)
+    blocked = 0
+    for h in [0, 17] + walkers[:: len(walkers) // 8].tolist():
+        offsets = {h: s.get_facet_offsets(h)}
+        nf, L = s.heliostat(h)["num_facets"], s.lights_per_group
+        want = o.trace([h], dirs, pert, offsets, record=(h, 0, nf), images=False)["records"]
+        s.set_math_mode(1)
+        got = s.hit_records(h, 0, nf, 0, L)
+        assert np.array_equal(got, want), f"heliostat {h} (code {codes[h]}): {np.mean(got != want):.2e} differ"
+        s.set_math_mode(0)
+        fast = s.hit_records(h, 0, nf, 0, L)
+        assert np.count_nonzero((fast >= 0) != (want >= 0)) <= 1 + 1e-4 * len(want)
+        blocked += int(np.sum(want == -2))
+    assert blocked > 0
+
+
 def test_sharded_trace_one_rank_equals_plain(small):
     """shard.ShardedTrace over a one-rank NCCL group: the collectives run on
     the tracer's own device image (a zero-copy view) and give the plain trace."""
