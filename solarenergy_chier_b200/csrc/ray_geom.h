@@ -22,10 +22,11 @@ __device__ __forceinline__ float3 xyz(float4 v) { return make_float3(v.x, v.y, v
 // acos takes its argument clamped to [-1, 1]; the reference prints an error
 // and lets a NaN through when rounding pushes it outside.
 __device__ __forceinline__ bool cylinder_hit(const DevReceiver& r, float3 o, float3 d, float& t, float& u, float& v) {
-  float2 l = make_float2(qm_rn_sub(o.x, r.pos.x), qm_rn_sub(o.z, r.pos.z));
+  // pos - o (the reference also forms o - pos, its exact negative)
+  const float2 ro = make_float2(qm_rn_sub(r.pos.x, o.x), qm_rn_sub(r.pos.z, o.z));
+  const float ro2 = qs::dot2(ro, ro);
   const float r2 = qm_rn_mul(r.size.x, r.size.x);
-  if (qs::dot2(l, l) <= r2) return false;
-  float2 ro = make_float2(qm_rn_sub(r.pos.x, o.x), qm_rn_sub(r.pos.z, o.z));
+  if (ro2 <= r2) return false;
   // The horizontal direction's squared length D, its correctly rounded
   // 1/sqrt and sqrt (normalize2 and length2 of the reference's test): for
   // D in [2^-100, 2^125) -- every ray but a vertical one -- from the series
@@ -44,7 +45,7 @@ __device__ __forceinline__ bool cylinder_hit(const DevReceiver& r, float3 o, flo
     tp = qs::dot2(ro, qs::normalize2(dxz));
     len = sqrtf(D);
   }
-  float delta = qm_rn_sub(qs::dot2(ro, ro), qm_rn_mul(tp, tp));
+  float delta = qm_rn_sub(ro2, qm_rn_mul(tp, tp));
   if (qm_below_neg_eps(tp) || delta > r2) return false;
   float t_plus = delta <= 0.0f ? r.size.x : sqrtf(qm_rn_sub(r2, delta));
   const float num = qm_rn_sub(tp, t_plus);

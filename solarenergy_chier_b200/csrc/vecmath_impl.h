@@ -28,7 +28,9 @@ QM_HD float3 normalize(float3 v) { float inv = rlen(dot(v, v)); return mul(v, in
 // normalize for vectors of unit scale (squared length in [2^-125, 2^125) or
 // NaN): the same value without the reciprocal square root's range test (QRU).
 QM_HD float3 normalize_unit(float3 v) { float inv = QRU(dot(v, v)); return mul(v, inv); }
-QM_HD float3 reflect(float3 i, float3 n) { return sub(i, mul(mul(n, 2.0f), dot(n, i))); }
+// The reference scales n by 2, then by the dot product; doubling is exact, so
+// doubling the dot product instead gives the same products.
+QM_HD float3 reflect(float3 i, float3 n) { return sub(i, mul(n, QM(2.0f, dot(n, i)))); }
 
 QM_HD float dot2(float2 a, float2 b) { return QA(QM(a.x, b.x), QM(a.y, b.y)); }
 QM_HD float length2(float2 v) { return sqrtf(dot2(v, v)); }
