@@ -485,7 +485,7 @@ int chunk_iters_for(int mode, int shape, int out, long long rays) {
 }
 
 cudaError_t launch_trace_mode(int mode, const qm::TraceParams& p, int out, cudaStream_t st, int shape, int chunk_iters,
-                              unsigned long long* work_counter) {
+                              unsigned long long* work_counter, const qm::CopiedImages& images) {
   cudaError_t e;
   switch (mode) {
     case 1: e = qm::launch_trace_exact(p, out, st, nullptr, chunk_iters); break;
@@ -495,7 +495,7 @@ cudaError_t launch_trace_mode(int mode, const qm::TraceParams& p, int out, cudaS
     default: e = kShapes[shape_for(mode, shape, out)].launch(p, out, st, work_counter, chunk_iters); break;
   }
   // flux and bilinear-deposit launches add their per-chunk power partials
-  if (e == cudaSuccess && (out == 0 || out == 2) && p.chunk_power) e = qm::launch_power_reduce(p, st);
+  if (e == cudaSuccess && (out == 0 || out == 2)) e = qm::launch_trace_end(p, images, st);
   return e;
 }
 
@@ -503,6 +503,50 @@ double* chunk_power_buffer(DBuf& buf, long long chunks) {
   const size_t need = (size_t)std::max<long long>(chunks, 1) * sizeof(double);
   if (buf.bytes < need) buf.alloc(need);
   return buf.as<double>();
+}
+
+// Deposits onto a small image crowd into few pixels, whose L2 slices then
+// bound the launch (on 160 x 120 pixels the busiest slice's atomic unit was
+// 68 % busy, the average 15 %); spread over 8 copies of the image, merged by
+// the launch that sums the power, they do not: 655 M rays of 50 heliostats
+// 9.3 -> 6.6 ms, 1.6 M rays of one 39 -> 31 us with its merge, but 1.3 M of 50
+// 35 -> 37 and 0.4 M of one 17 -> 21, hence from 1.5 M rays on.  On the 754,200 pixels of the
+// 624-heliostat field the slices share the load (13 and 19 %); the largest
+// image that is copied keeps its copies in 4 MiB.
+constexpr int kImageCopies = 8;
+constexpr long long kCopiedPixels = 1 << 17;
+constexpr long long kCopiedRays = 1500 * 1000;
+
+// The scene's copies, made at the first launch that uses them; whether any
+// of the receivers of heliostats ids[0..n) has some.
+bool image_copies(qmcrt_scene* s, const int* ids, int n) {
+  auto small = [&](const DevReceiver& r) { return (long long)r.resolution.x * r.resolution.y <= kCopiedPixels; };
+  bool used = false;
+  for (int i = 0; i < n && !used; ++i) used = small(s->receivers[s->templates[ids[i]].receiver]);
+  if (!used || s->copies_ready) return used;
+  std::vector<DevReceiver> recv = s->receivers;
+  auto stride = [](const DevReceiver& r) { return (r.resolution.x * r.resolution.y + 31) / 32 * 32; };
+  size_t floats = 0;
+  int count = 0;
+  for (const auto& r : recv)
+    if (small(r) && count++ < qm::kMaxCopiedImages) floats += (size_t)kImageCopies * stride(r);
+  s->d_copy_receivers.alloc(recv.size() * sizeof(DevReceiver));
+  s->d_copies.alloc(floats * sizeof(float));
+  cuda_check(cudaMemset(s->d_copies.p, 0, floats * sizeof(float)), "cudaMemset");
+  cuda_check(cudaDeviceSynchronize(), "image copies");
+  s->copied.n = 0;
+  float* next = s->d_copies.as<float>();
+  for (auto& r : recv) {
+    if (!small(r) || s->copied.n == qm::kMaxCopiedImages) continue;
+    s->copied.at[s->copied.n++] = {r.image, next, r.resolution.x * r.resolution.y, kImageCopies, stride(r)};
+    r.image = next;
+    r.copy_mask = kImageCopies - 1;
+    r.copy_stride = stride(r);
+    next += (size_t)kImageCopies * stride(r);
+  }
+  upload(s->d_copy_receivers, recv);
+  s->copies_ready = true;
+  return used;
 }
 
 // Traces heliostats ids[0..n) over the scene's light range: out 0 adds their
@@ -592,7 +636,11 @@ long long trace_ids(qmcrt_scene* s, const int* ids, int n, cudaStream_t stream, 
     if (s->d_work.bytes < sizeof(unsigned long long)) s->d_work.alloc(sizeof(unsigned long long));
     work = s->d_work.as<unsigned long long>();
   }
-  cuda_check(launch_trace_mode(s->exact, p, out, stream, s->shape, chunk_iters, work), "trace kernel");
+  const bool copied = out == 0 && rays >= kCopiedRays && image_copies(s, ids, n);
+  if (copied) p.receivers = s->d_copy_receivers.as<DevReceiver>();
+  cuda_check(launch_trace_mode(s->exact, p, out, stream, s->shape, chunk_iters, work,
+                               copied ? s->copied : qm::CopiedImages()),
+             "trace kernel");
   return total;
 }
 

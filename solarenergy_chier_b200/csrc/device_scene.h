@@ -51,6 +51,9 @@ struct DevReceiver {
   float3 a, ab, ac;     // rectangle: vertex 0, v1 - v0, v3 - v0
   float3 pos, size;     // cylinder: centre, (radius, height, -)
   float rcp_height;     // cylinder: 1 / height rounded to nearest (host division)
+  // Flux launches: block b deposits into copy (b & copy_mask) of the image,
+  // copy_stride floats apart (0, 0: the image alone).
+  int copy_mask, copy_stride;
 };
 
 // One heliostat to trace (a HeliostatArgument plus the per-heliostat

@@ -5,7 +5,7 @@
 // rays' energies: per-lane sums of at most 64 float energies, exact in
 // double for the magnitudes of one heliostat, then a warp shuffle tree) to
 // TraceParams::chunk_power.  This kernel adds each task's partials, one warp
-// or one block of 8 warps per task: every lane runs a Neumaier-compensated
+// or one block of 8 or 32 warps per task: every lane runs a Neumaier-compensated
 // sum over a strided subset, the 32 (sum, compensation) pairs of a warp merge
 // by error-free two-sums down a fixed shuffle tree, the warps' pairs likewise
 // in warp order, and lane 0 adds the rounded result to the task's power slot.
@@ -33,12 +33,36 @@ __device__ __forceinline__ void merge(double& s, double& c, double s2, double c2
   s = sum;
 }
 
+// Pixels of the copied images, one per thread of the launch's later blocks.
+// Every value is taken and zeroed by one exchange, so a deposit that another
+// stream's launch makes meanwhile is counted here or by its own merge.
+__device__ __forceinline__ void merge_copies(const CopiedImages& images, long long i) {
+  for (int r = 0; r < images.n; ++r) {
+    const CopiedImage& m = images.at[r];
+    if (i >= m.pixels) {
+      i -= m.pixels;
+      continue;
+    }
+    float s = 0.0f;
+#pragma unroll 8
+    for (int k = 0; k < m.copies_n; ++k) s += atomicExch(m.copies + (size_t)k * m.stride + i, 0.0f);
+    if (s != 0.0f) atomicAdd(m.image + i, s);
+    return;
+  }
+}
+
 // A task's partials are a chain of loads and dependent adds per lane, so the
-// kernel's time is its longest chain: kWarps = 8 shortens it for tasks of
-// many chunks, where a warp alone would take hundreds of steps.
+// kernel's time is its longest chain: 8 or 32 warps shorten it for tasks of
+// many chunks, where a warp alone would take hundreds of steps.  Blocks from
+// power_blocks on merge the copied images, in the same launch.
 template <int kWarps>
-__global__ void __launch_bounds__(128 * (kWarps > 4 ? kWarps / 4 : 1)) power_reduce_kernel(TraceParams p) {
+__global__ void __launch_bounds__(kWarps > 4 ? 32 * kWarps : 128)
+    power_reduce_kernel(TraceParams p, CopiedImages images, int power_blocks) {
   __shared__ double part[kWarps][2];
+  if ((int)blockIdx.x >= power_blocks) {
+    merge_copies(images, (long long)(blockIdx.x - power_blocks) * blockDim.x + threadIdx.x);
+    return;
+  }
   const int lane = threadIdx.x & 31, warp = kWarps > 1 ? threadIdx.x >> 5 : 0;
   const long long t = kWarps > 1 ? blockIdx.x : ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (t >= p.num_tasks) return;
@@ -77,16 +101,24 @@ __global__ void __launch_bounds__(128 * (kWarps > 4 ? kWarps / 4 : 1)) power_red
 
 }  // namespace
 
-cudaError_t launch_power_reduce(const TraceParams& p, cudaStream_t stream) {
-  if (!p.chunk_power || p.num_tasks <= 0) return cudaSuccess;
-  // 8 warps per task from 256 chunks a task on: one step per lane (a lone
-  // heliostat of 1,600 chunks: 50 steps of a warp or 7 of 8 warps).
-  if ((p.total_facets - p.chunk_begin) / p.num_tasks >= 256) {
-    power_reduce_kernel<8><<<(unsigned)p.num_tasks, 256, 0, stream>>>(p);
-  } else {
-    const int threads = 128;
-    const long long blocks = ((long long)p.num_tasks * 32 + threads - 1) / threads;
-    power_reduce_kernel<1><<<(unsigned)blocks, threads, 0, stream>>>(p);
+cudaError_t launch_trace_end(const TraceParams& p, const CopiedImages& images, cudaStream_t stream) {
+  const bool power = p.chunk_power && p.num_tasks > 0;
+  long long pixels = 0;
+  for (int r = 0; r < images.n; ++r) pixels += images.at[r].pixels;
+  if (!power && pixels == 0) return cudaSuccess;
+  // 8 warps per task from 256 chunks a task on (one step per lane), 32 from
+  // 1,024: a lone heliostat of 6,400 chunks takes 7 steps of 32 warps, where 8
+  // took 25 and a warp alone 200.
+  const long long per_task = power ? (p.total_facets - p.chunk_begin) / p.num_tasks : 0;
+  const int warps = per_task >= 1024 ? 32 : (per_task >= 256 ? 8 : 1);
+  const int threads = warps > 1 ? 32 * warps : 128;
+  const int power_blocks = !power ? 0 : (int)(warps > 1 ? p.num_tasks : ((long long)p.num_tasks * 32 + 127) / 128);
+  const long long blocks = power_blocks + (pixels + threads - 1) / threads;
+  if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+  switch (warps) {
+    case 32: power_reduce_kernel<32><<<(unsigned)blocks, threads, 0, stream>>>(p, images, power_blocks); break;
+    case 8: power_reduce_kernel<8><<<(unsigned)blocks, threads, 0, stream>>>(p, images, power_blocks); break;
+    default: power_reduce_kernel<1><<<(unsigned)blocks, threads, 0, stream>>>(p, images, power_blocks); break;
   }
   return cudaGetLastError();
 }

@@ -402,6 +402,7 @@ struct FacetWindow {
   // g in [0, P) plus a light index in [0, L) needs no wrap-around).
   const float4* samples[kThreads / 32];
   const float4* perturbations[kThreads / 32];
+  float* image[kThreads / 32];     // where the warp's flux goes (DevReceiver::copy_mask)
   int shadow_free[kThreads / 32];  // the task's shadow-walk code (DevTask::shadow_free)
   float4 o[kThreads];   // origin.xyz, pool offset g[f] (int bits)
   float4 u[kThreads];   // frame u.xyz, pool offset g[(f+1) % P] (int bits; bit 31: block walk skippable)
@@ -431,6 +432,10 @@ __device__ __forceinline__ const float4* lds_ptr(const float4* const& x) {
   const unsigned a = (unsigned)__cvta_generic_to_shared(&x);
   asm volatile("ld.shared.u64 %0, [%1];" : "=l"(r) : "r"(a));
   return reinterpret_cast<const float4*>(r);
+}
+
+__device__ __forceinline__ float* lds_image(float* const& x) {
+  return const_cast<float*>(reinterpret_cast<const float*>(lds_ptr(reinterpret_cast<const float4* const&>(x))));
 }
 
 // DDA start of a facet's walks, computed from its origin when a ray walks
@@ -528,6 +533,7 @@ __global__ void __launch_bounds__(kThreads, QM_TRACE_MIN_BLOCKS) trace_kernel(QM
   const DevReceiver& R = p.receivers[T.receiver];
   if (lane == 0) {
     win.shadow_free[threadIdx.x >> 5] = T.shadow_free;
+    win.image[threadIdx.x >> 5] = R.image + (size_t)(blockIdx.x & R.copy_mask) * R.copy_stride;
     win.samples[threadIdx.x >> 5] = T.samples;
     win.perturbations[threadIdx.x >> 5] = T.perturbations;
   }
@@ -648,13 +654,13 @@ __global__ void __launch_bounds__(kThreads, QM_TRACE_MIN_BLOCKS) trace_kernel(QM
             } else {
             int row = int(QM_PIXEL_MUL(uu, (float)R.resolution.y));
             int col = int(QM_PIXEL_MUL(vv, (float)R.resolution.x));
-            if (row >= R.resolution.y || col >= R.resolution.x || row < 0 || col < 0) {
+            if ((unsigned)row >= (unsigned)R.resolution.y || (unsigned)col >= (unsigned)R.resolution.x) {
               row = min(max(row, 0), R.resolution.y - 1);
               col = min(max(col, 0), R.resolution.x - 1);
               ++clamped;
             }
             const int pix = row * R.resolution.x + col;
-            atomicAdd(R.image + pix, e);
+            atomicAdd(lds_image(win.image[threadIdx.x >> 5]) + pix, e);
             power += (double)e;
             code = pix;
             }

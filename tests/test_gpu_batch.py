@@ -154,6 +154,36 @@ def test_chunk_sizes_of_small_launches(heliostats, lights, tmp_path):
     np.testing.assert_allclose(p, p0, rtol=1e-12, atol=0)
 
 
+@pytest.mark.parametrize("mode", [0, 1])
+def test_image_copies_of_small_receivers(mode, tmp_path):
+    """Flux launches of 1.5 M rays and more onto small receivers deposit
+    through copies of the images: one launch gives what smaller launches over
+    the same lights add up to directly (L1 <= 1e-6, FP64 powers 1e-12), on
+    both receivers of a scene, a second launch adds to the images, and
+    nothing is left in the copies."""
+    f = synth.two_receiver_field(tmp_path, seed=1, helio_pixel=0.05, groups=4, per_group=128)
+    s = q.Scene(f.scene, f.config, device=0, seed=2)
+    s.set_math_mode(mode)
+    ids = list(range(s.num_heliostats))
+    facets = sum(s.heliostat(h)["num_facets"] for h in ids)
+    assert 4 * facets < 1.5e6 <= 12 * facets
+
+    def traced(ranges):
+        s.clear()
+        s.clear_power()
+        for r in ranges:
+            s.set_light_range(*r)
+            s.trace(ids)
+        return [s.image(k).astype(np.float64) for k in (0, 1)], s.power()[0]
+
+    pieces, p0 = traced([(3, 7), (7, 11), (11, 15)])
+    for times in (1, 2):
+        images, p = traced([(3, 15)] * times)
+        for a, b in zip(images, pieces):
+            assert b.sum() > 0 and np.abs(a - times * b).sum() <= 1e-6 * times * b.sum()
+        np.testing.assert_allclose(p, times * p0, rtol=1e-12, atol=0)
+
+
 def test_every_launch_shape_gives_the_same_result(fields, tmp_path):
     """The autotuner's candidates (launch shapes of the production build:
     block widths, warp chunks of 32, 64 or 128 iterations) change only how
