@@ -109,7 +109,8 @@ __global__ void shadow_kernel(PrepInputs p, int max_sub, const DevGrid* grids) {
   const SunParams& sun = p.suns[it.sun];
   DevTask& T = p.tasks[it.task];
   const DevGrid& G = grids[T.grid];
-  const ShadowGrid view{G.pos, G.interval, G.cells, G.bound, G.cell_range, G.entries};
+  const ShadowGrid view{G.pos,       G.interval, G.cells, G.bound, G.cell_range, G.entries,
+                        __int_as_float(height_key(G.top_key))};
   Cone cone;
   if (slot == 0) {
     const int state = sun.shadow_tan >= 0.0f ? shadow_cone(view, T.own, sun.shadow_axis, sun.shadow_tan, cone) : -1;

@@ -30,6 +30,7 @@ struct ShadowGrid {
   const float4* bound;    // 5 float4 per grid-local heliostat (centre, then axes with half extents)
   const int2* ranges;     // [begin, end) of each cell's entries
   const int4* entries;    // grid-local heliostat id first
+  float top;              // highest point of the padded boxes
 };
 
 // Ray (o, a) against the box of record b widened by w on every axis: true
@@ -73,17 +74,23 @@ QM_HD int make_cone(const ShadowGrid& g, float3 c, float ri, float3 axis, float 
   const float3 a = make_float3(axis.x / al, axis.y / al, axis.z / al);
   const float tq = tan_theta * sqrtf(1.0f + tan_theta * tan_theta) * 1.001f + 1e-6f;
   const float margin = 0.05f + 2e-6f * (fabsf(c.x) + fabsf(c.y) + fabsf(c.z));
+  // Rays can hit something inside the grid and below the highest box only.
   const float3 lo = g.pos;
-  const float3 hi = make_float3(g.pos.x + g.cells.x * g.interval.x, g.pos.y + g.cells.y * g.interval.y,
-                                g.pos.z + g.cells.z * g.interval.z);
+  float3 hi = make_float3(g.pos.x + g.cells.x * g.interval.x, g.pos.y + g.cells.y * g.interval.y,
+                          g.pos.z + g.cells.z * g.interval.z);
+  if (g.top + margin < hi.y) hi.y = g.top + margin;
   const float dx = hi.x - lo.x, dy = hi.y - lo.y, dz = hi.z - lo.z;
-  // Longest axis run that can matter: inside the grid widened by the widest
-  // capsule radius.
-  const float s_max = sqrtf(dx * dx + dy * dy + dz * dz) + 4.0f * ri + 10.0f;
-  const float R = ri + (s_max + ri) * tq + margin;
-  float s_end = s_max;
-  {
-    // where the axis leaves the grid widened by R
+  // Axis run that can matter, and the widest capsule radius on it: first the
+  // longest line in that region, then what is left while the axis is inside
+  // the region widened by the radius reached so far (rays within s_end are
+  // within R of the axis, so those inside the region leave it where the axis
+  // leaves the widened one).  Three rounds bring a flat cone over a wide grid
+  // from the grid's diagonal near the run where its lower edge passes the
+  // mirrors' tops.
+  float s_end = sqrtf(dx * dx + dy * dy + dz * dz) + 4.0f * ri + 10.0f;
+  float R = 0.0f;
+  for (int round = 0; round < 3; ++round) {
+    R = ri + (s_end + ri) * tq + margin;
     float tn = -3.0e38f, tf = 3.0e38f;
     const float ov[3] = {c.x, c.y, c.z}, dv[3] = {a.x, a.y, a.z};
     const float lv[3] = {lo.x - R, lo.y - R, lo.z - R}, hv[3] = {hi.x + R, hi.y + R, hi.z + R};
@@ -99,6 +106,7 @@ QM_HD int make_cone(const ShadowGrid& g, float3 c, float ri, float3 axis, float 
     if (tf < -ri) return 0;
     s_end = fminf(s_end, tf);
   }
+  R = ri + (s_end + ri) * tq + margin;
   const float s0 = -ri;
   const float3 p0 = make_float3(c.x + s0 * a.x, c.y + s0 * a.y, c.z + s0 * a.z);
   const float3 p1 = make_float3(c.x + s_end * a.x, c.y + s_end * a.y, c.z + s_end * a.z);
@@ -140,9 +148,10 @@ QM_HD bool cone_meets(const Cone& o, const float4* bj) {
 // tests that cell's entries; the few that meet the cone are merged by the
 // warp one at a time.  The enumeration is a chain of dependent loads (cell
 // range -> entry -> record), so a thread that ran a cone alone paid a latency
-// per entry; spread over a warp it pays one per 32 cells.  A sun of the
-// 648-heliostat field (3,240 cones): 977 -> 42 us; 12 suns of 156 focus-flat
-// and 692 flat heliostats (70,900 cones): 1,488 -> 536 us.
+// per entry; spread over a warp it pays one per 32 cells.  12 suns of 156
+// focus-flat and 692 flat heliostats (70,900 cones): 1,488 -> 536 us, and 207
+// with the cone's run bounded by the mirrors' tops (make_cone); 4 suns of
+// 10,000 flat ones (80,000 cones): 9,908, 2,166 and 224 us.
 __device__ __forceinline__ int warp_candidates(const ShadowGrid& g, int own, const Cone& o, int cap, int& found) {
   const int lane = threadIdx.x & 31;
   const int nx = o.hi[0] - o.lo[0] + 1, ny = o.hi[1] - o.lo[1] + 1, nz = o.hi[2] - o.lo[2] + 1;

@@ -56,7 +56,12 @@ int main(int argc, char** argv) {
         qm::heliostat_record(&g.sub_vertices[3 * (size_t)h.sub_begin], h.num_sub, h.row_col, h.pos, h.normal,
                              &bound[5 * (size_t)i], &rc);
       }
-      const qm::ShadowGrid view{g.pos, g.interval, g.cells, bound.data(), ranges.data(), entries.data()};
+      float top = -3.0e38f;
+      for (size_t i = 0; i < bound.size(); i += 5) {
+        const float4* c = &bound[i];
+        top = std::fmax(top, c[0].y + std::fabs(c[1].y) * c[1].w + std::fabs(c[2].y) * c[2].w + std::fabs(c[3].y) * c[3].w);
+      }
+      const qm::ShadowGrid view{g.pos, g.interval, g.cells, bound.data(), ranges.data(), entries.data(), top};
       qm::Cone o;
       for (int i = 0; i < g.num_heliostats; ++i) {
         const auto& h = m.heliostats[g.start_heliostat + i];
