@@ -59,6 +59,8 @@ template <int kWarps>
 __global__ void __launch_bounds__(kWarps > 4 ? 32 * kWarps : 128)
     power_reduce_kernel(TraceParams p, CopiedImages images, int power_blocks) {
   __shared__ double part[kWarps][2];
+  wait_previous();
+  begin_next();
   if ((int)blockIdx.x >= power_blocks) {
     merge_copies(images, (long long)(blockIdx.x - power_blocks) * blockDim.x + threadIdx.x);
     return;
@@ -116,11 +118,10 @@ cudaError_t launch_trace_end(const TraceParams& p, const CopiedImages& images, c
   const long long blocks = power_blocks + (pixels + threads - 1) / threads;
   if (blocks > 0x7fffffffLL) return cudaErrorInvalidValue;
   switch (warps) {
-    case 32: power_reduce_kernel<32><<<(unsigned)blocks, threads, 0, stream>>>(p, images, power_blocks); break;
-    case 8: power_reduce_kernel<8><<<(unsigned)blocks, threads, 0, stream>>>(p, images, power_blocks); break;
-    default: power_reduce_kernel<1><<<(unsigned)blocks, threads, 0, stream>>>(p, images, power_blocks); break;
+    case 32: return launch_overlapped(power_reduce_kernel<32>, (unsigned)blocks, threads, stream, p, images, power_blocks);
+    case 8: return launch_overlapped(power_reduce_kernel<8>, (unsigned)blocks, threads, stream, p, images, power_blocks);
+    default: return launch_overlapped(power_reduce_kernel<1>, (unsigned)blocks, threads, stream, p, images, power_blocks);
   }
-  return cudaGetLastError();
 }
 
 }  // namespace qm

@@ -493,6 +493,8 @@ template <int kOut, int kIters = kChunkIters>
 #endif
 __global__ void __launch_bounds__(kThreads, QM_TRACE_MIN_BLOCKS) trace_kernel(QM_TRACE_ARGS) {
   __shared__ FacetWindow win;
+  wait_previous();
+  begin_next();
   const int lane = threadIdx.x & 31;
   const int wbase = threadIdx.x & ~31;  // this warp's 32 window slots
 #if defined(QM_TRACE_PERSISTENT)
@@ -778,12 +780,10 @@ cudaError_t QM_SYM(launch_trace)(const TraceParams& params, int out, cudaStream_
     default:
 #if QM_CHUNK_ITERS == 64 && QM_TRACE_THREADS != 64 && !defined(QM_TRACE_PERSISTENT)
       if (chunk_iters == kSmallChunkIters) {
-        trace_kernel<kOutFlux, kSmallChunkIters><<<(unsigned)blocks, threads, 0, stream>>>(QM_TRACE_LAUNCH_ARGS);
-        break;
+        return launch_overlapped(trace_kernel<kOutFlux, kSmallChunkIters>, (unsigned)blocks, threads, stream, p);
       }
       if (chunk_iters == kMediumChunkIters) {
-        trace_kernel<kOutFlux, kMediumChunkIters><<<(unsigned)blocks, threads, 0, stream>>>(QM_TRACE_LAUNCH_ARGS);
-        break;
+        return launch_overlapped(trace_kernel<kOutFlux, kMediumChunkIters>, (unsigned)blocks, threads, stream, p);
       }
 #endif
       if (chunk_iters != kChunkIters) return cudaErrorInvalidValue;
