@@ -262,8 +262,10 @@ struct Facet {
   int g0, g1;
 };
 
-// The values follow the dual arithmetic of the preparation (value parts).
-__device__ __forceinline__ Facet make_facet(const DevTask& T, const DiffTask& DT, int f) {
+// The values follow the dual arithmetic of the preparation (value parts).  Not
+// inlined: once per 32 facets, beside a sweep whose code the one-warp blocks
+// of an SM, each at another place in it, must hold in one instruction cache.
+__device__ __noinline__ Facet make_facet(const DevTask& T, const DiffTask& DT, int f) {
   Facet fd;
   const bool focus_flat = facet_local(T, f, fd.local, fd.local_normal);
   DFrameT<0> hf;
@@ -463,7 +465,7 @@ __device__ __forceinline__ void ray_adjoint(const ChunkConstants& T, const Facet
 #define QM_BWD_THREADS 32
 #endif
 #ifndef QM_BWD_MIN_BLOCKS
-#define QM_BWD_MIN_BLOCKS 20
+#define QM_BWD_MIN_BLOCKS 24
 #endif
 constexpr int kBwdThreads = QM_BWD_THREADS;
 constexpr int kFacetFloats = 18;
@@ -483,13 +485,16 @@ __device__ __forceinline__ float3 get3(const AdjointWindow& w, int first, int sl
   return make_float3(w.value[first][slot], w.value[first + 1][slot], w.value[first + 2][slot]);
 }
 
-// Bound by instruction issue (69 % of slots; 13.4 warp instructions a ray).
-// Run backwards a ray costs its value chain, one sweep of vector adjoints and
-// 18 multiply-adds into the frame sums, against four tangents through every
-// operation (33 warp instructions a ray); the queue gives every sweep 32 hits
-// where a chunk's iterations hold 22 on the benchmark field.  462 M rays, 32
-// lights per facet: 17.9 -> 7.8 ms (11.7 of it before the shared constants and
-// the four-pixel read); 256 M rays, 4 lights: 11.9 -> 6.6.
+// Bound by instruction issue (76 % of the slots; 15.5 warp instructions a ray
+// at 8 lights per facet, 13.4 at 32).  Run backwards a ray costs its value chain, one
+// sweep of vector adjoints and 18 multiply-adds into the frame sums, against
+// four tangents through every operation (34 warp instructions a ray); the
+// queue gives every sweep 32 hits where a chunk's iterations hold 22 on the
+// benchmark field.  462 M rays, 32 lights per facet: 17.9 -> 7.4 ms (11.7 of it
+// before the shared constants and the four-pixel read, 7.8 before the sweep
+// stood in the code once and the facets apart from it: 15 % of the stalls
+// waited for instructions); 256 M rays, 4 lights: 11.9 -> 5.5, 6.6 before that.
+// 20 / 24 / 28 blocks per SM: 8.2 / 7.9 / 8.3 ms with the facets still inlined.
 __global__ void __launch_bounds__(kBwdThreads, QM_BWD_MIN_BLOCKS) diff_backward_kernel(BackwardParams p) {
   __shared__ AdjointWindow win;
   const int lane = threadIdx.x & 31;
@@ -516,40 +521,43 @@ __global__ void __launch_bounds__(kBwdThreads, QM_BWD_MIN_BLOCKS) diff_backward_
   FrameSum sum{};
   int base = 0;
   bool filled = false;  // warp-uniform
-  int queued = 0;       // warp-uniform, below 32 between iterations
+  int queued = 0;       // warp-uniform, at most 63
   int* q_slot = win.slot + 2 * wbase;
   int* q_light = win.light + 2 * wbase;
-  // Runs the last n <= 32 queued hits, one per lane.
-  auto run = [&](int n) {
-    __syncwarp();
-    if (lane < n) {
-      const int slot = q_slot[queued - n + lane], light = q_light[queued - n + lane];
-      Facet fd;
-      fd.origin = get3(win, 0, slot);
-      fd.u = get3(win, 3, slot);
-      fd.n = get3(win, 6, slot);
-      fd.v = get3(win, 9, slot);
-      fd.local = get3(win, 12, slot);
-      fd.local_normal = get3(win, 15, slot);
-      fd.identity = win.identity[slot] != 0;
-      fd.g0 = win.g0[slot];
-      fd.g1 = win.g1[slot];
-      ray_adjoint(win.shared[threadIdx.x >> 5], fd, light, sum);
-    }
-    queued -= n;
-    __syncwarp();
-  };
   unsigned words = 0;  // lane i: hit bits of iteration 32 (it / 32) + i
-  for (int it = 0; it < iters; ++it) {
+  for (int it = 0;; ++it) {
+    const bool more = it < iters;  // a last step runs what still waits
     if ((it & 31) == 0) words = it + lane < iters ? __ldg(p.hit_bits + warp * kChunkIters + it + lane) : 0u;
     const unsigned bits = __shfl_sync(0xffffffffu, words, it & 31);
-    const bool hit = r0 + it * 32 + lane < r_end && ((bits >> lane) & 1u);
+    const bool hit = more && r0 + it * 32 + lane < r_end && ((bits >> lane) & 1u);
     // The facets of an iteration lie within 32 of lane 0's (see the trace
     // kernel); refill the window when a lane with a hit needs one past it,
     // after the hits that are waiting with the present one.
     const int f0 = __shfl_sync(0xffffffffu, f, 0);
-    if (__any_sync(0xffffffffu, hit && (!filled || f - base >= 32))) {
-      if (queued > 0) run(queued);
+    const bool fill = __any_sync(0xffffffffu, hit && (!filled || f - base >= 32));
+    // Runs the last queued hits, one per lane, at this one place in the code.
+    while (fill || !more ? queued > 0 : queued >= 32) {
+      const int n = min(queued, 32);
+      __syncwarp();
+      if (lane < n) {
+        const int slot = q_slot[queued - n + lane], light = q_light[queued - n + lane];
+        Facet fd;
+        fd.origin = get3(win, 0, slot);
+        fd.u = get3(win, 3, slot);
+        fd.n = get3(win, 6, slot);
+        fd.v = get3(win, 9, slot);
+        fd.local = get3(win, 12, slot);
+        fd.local_normal = get3(win, 15, slot);
+        fd.identity = win.identity[slot] != 0;
+        fd.g0 = win.g0[slot];
+        fd.g1 = win.g1[slot];
+        ray_adjoint(win.shared[threadIdx.x >> 5], fd, light, sum);
+      }
+      queued -= n;
+      __syncwarp();
+    }
+    if (!more) break;
+    if (fill) {
       __syncwarp();
       base = f0;
       filled = true;
@@ -575,7 +583,6 @@ __global__ void __launch_bounds__(kBwdThreads, QM_BWD_MIN_BLOCKS) diff_backward_
       q_light[k] = p.light_begin + l;
     }
     queued += __popc(hits);
-    if (queued >= 32) run(32);
     f += p.lights_q32;
     l += p.lights_r32;
     if (l >= nl) {
@@ -583,7 +590,6 @@ __global__ void __launch_bounds__(kBwdThreads, QM_BWD_MIN_BLOCKS) diff_backward_
       ++f;
     }
   }
-  if (queued > 0) run(queued);
   // d(axes)/d(parameters) of the heliostat's facet frame; constant axes when
   // the frame is the identity.
   if (DT.identity) return;
