@@ -160,6 +160,41 @@ void model_for_sun(const qmcrt_scene* s) {
   s->model_stale = false;
 }
 
+// The largest image that has a spread one (see kSpreadRays), 4.5 MiB of it.
+constexpr long long kSpreadPixels = 1 << 17;
+bool spread_pixels(const DevReceiver& r) { return (long long)r.resolution.x * r.resolution.y <= kSpreadPixels; }
+
+// The scene's receivers, and a second time with the spread images that are
+// made here for the small ones.
+std::vector<DevReceiver> with_spread_images(qmcrt_scene* s) {
+  std::vector<DevReceiver> recv = s->receivers;
+  s->spread.n = 0;
+  s->d_spread.release();
+  if (recv.size() <= (size_t)qm::kMaxSpreadImages) {
+    size_t floats = 0;
+    for (auto& r : s->receivers) {
+      if (spread_pixels(r)) {
+        const int pixels = r.resolution.x * r.resolution.y;
+        s->spread.at[s->spread.n++] = {r.image, nullptr, pixels, qm::kImageSpread};
+        floats += (size_t)pixels * qm::kImageSpread;
+      }
+      recv.push_back(r);
+    }
+    if (floats) {
+      s->d_spread.alloc(floats * sizeof(float));
+      cuda_check(cudaMemset(s->d_spread.p, 0, s->d_spread.bytes), "cudaMemset");
+    }
+    float* next = s->d_spread.as<float>();
+    int k = 0;
+    for (size_t r = s->receivers.size(); r < recv.size(); ++r) {
+      if (!spread_pixels(recv[r])) continue;
+      s->spread.at[k++].spread = recv[r].image = next;
+      next += (size_t)recv[r].resolution.x * recv[r].resolution.y * qm::kImageSpread;
+    }
+  }
+  return recv;
+}
+
 void build_device_scene(qmcrt_scene* s) {
   qm::SceneModel& m = s->model;
   const qm::SceneConfig& cfg = m.config;
@@ -241,7 +276,7 @@ void build_device_scene(qmcrt_scene* s) {
     s->receivers.push_back(dr);
     s->images.push_back(std::move(img));
   }
-  upload(s->d_receivers, s->receivers);
+  upload(s->d_receivers, with_spread_images(s));
 
   // Focus-flat local facet frames.
   std::vector<float3> local;
@@ -485,7 +520,7 @@ int chunk_iters_for(int mode, int shape, int out, long long rays) {
 }
 
 cudaError_t launch_trace_mode(int mode, const qm::TraceParams& p, int out, cudaStream_t st, int shape, int chunk_iters,
-                              unsigned long long* work_counter, const qm::CopiedImages& images) {
+                              unsigned long long* work_counter, const qm::SpreadImages& images) {
   cudaError_t e;
   switch (mode) {
     case 1: e = qm::launch_trace_exact(p, out, st, nullptr, chunk_iters); break;
@@ -505,48 +540,29 @@ double* chunk_power_buffer(DBuf& buf, long long chunks) {
   return buf.as<double>();
 }
 
-// Deposits onto a small image crowd into few pixels, whose L2 slices then
+// Deposits onto a small image crowd into few sectors of L2, whose slices then
 // bound the launch (on 160 x 120 pixels the busiest slice's atomic unit was
-// 68 % busy, the average 15 %); spread over 8 copies of the image, merged by
-// the launch that sums the power, they do not: 655 M rays of 50 heliostats
-// 9.3 -> 6.6 ms, 1.6 M rays of one 39 -> 31 us with its merge, but 1.3 M of 50
-// 35 -> 37 and 0.4 M of one 17 -> 21, hence from 1.5 M rays on.  On the 754,200 pixels of the
-// 624-heliostat field the slices share the load (13 and 19 %); the largest
-// image that is copied keeps its copies in 4 MiB.
-constexpr int kImageCopies = 8;
-constexpr long long kCopiedPixels = 1 << 17;
-constexpr long long kCopiedRays = 1500 * 1000;
+// 68 % busy, the average 15 %).  Such launches deposit into a spread image,
+// one pixel per kImageSpread floats, into which a first launch moves the
+// image's values and from which the launch that sums the power moves them
+// back: still one float accumulator per pixel, so a pixel's rounding error
+// is what it was (8 copies of the image, merged, were 0.07 ms faster on 655 M
+// rays but 5e-5 from the sums of one accumulator).  655 M rays of 50
+// heliostats, ms at 1 / 2 / 4 / 6 / 8 / 9 / 12 / 16 / 32 floats a pixel:
+// 8.7 / 7.2 / 7.0 / 6.8 / 7.2 / 6.7 / 7.0 / 7.5 / 8.3: of the steps of a
+// sector and more the odd one does best.  Whole launches, us without / with: one heliostat, 0.4 M rays
+// 14 / 18, 1.6 M 34 / 30, 6.6 M 115 / 84; 50 of them, 1.3 M 32 / 33, 5.1 M
+// 79 / 73, 41 M 548 / 456, 164 M 2,172 / 1,679; hence from 1.5 M rays on.  On the
+// 754,200 pixels of the 624-heliostat field the slices share the load (13 and
+// 19 %).
+constexpr long long kSpreadRays = 1500 * 1000;
 
-// The scene's copies, made at the first launch that uses them; whether any
-// of the receivers of heliostats ids[0..n) has some.
-bool image_copies(qmcrt_scene* s, const int* ids, int n) {
-  auto small = [&](const DevReceiver& r) { return (long long)r.resolution.x * r.resolution.y <= kCopiedPixels; };
-  bool used = false;
-  for (int i = 0; i < n && !used; ++i) used = small(s->receivers[s->templates[ids[i]].receiver]);
-  if (!used || s->copies_ready) return used;
-  std::vector<DevReceiver> recv = s->receivers;
-  auto stride = [](const DevReceiver& r) { return (r.resolution.x * r.resolution.y + 31) / 32 * 32; };
-  size_t floats = 0;
-  int count = 0;
-  for (const auto& r : recv)
-    if (small(r) && count++ < qm::kMaxCopiedImages) floats += (size_t)kImageCopies * stride(r);
-  s->d_copy_receivers.alloc(recv.size() * sizeof(DevReceiver));
-  s->d_copies.alloc(floats * sizeof(float));
-  cuda_check(cudaMemset(s->d_copies.p, 0, floats * sizeof(float)), "cudaMemset");
-  cuda_check(cudaDeviceSynchronize(), "image copies");
-  s->copied.n = 0;
-  float* next = s->d_copies.as<float>();
-  for (auto& r : recv) {
-    if (!small(r) || s->copied.n == qm::kMaxCopiedImages) continue;
-    s->copied.at[s->copied.n++] = {r.image, next, r.resolution.x * r.resolution.y, kImageCopies, stride(r)};
-    r.image = next;
-    r.copy_mask = kImageCopies - 1;
-    r.copy_stride = stride(r);
-    next += (size_t)kImageCopies * stride(r);
-  }
-  upload(s->d_copy_receivers, recv);
-  s->copies_ready = true;
-  return used;
+// Whether the receivers of heliostats ids[0..n) all have spread images.
+bool spread_images(const qmcrt_scene* s, const int* ids, int n) {
+  if (s->spread.n == 0) return false;
+  for (int i = 0; i < n; ++i)
+    if (!spread_pixels(s->receivers[s->templates[ids[i]].receiver])) return false;
+  return true;
 }
 
 // Traces heliostats ids[0..n) over the scene's light range: out 0 adds their
@@ -636,10 +652,15 @@ long long trace_ids(qmcrt_scene* s, const int* ids, int n, cudaStream_t stream, 
     if (s->d_work.bytes < sizeof(unsigned long long)) s->d_work.alloc(sizeof(unsigned long long));
     work = s->d_work.as<unsigned long long>();
   }
-  const bool copied = out == 0 && rays >= kCopiedRays && image_copies(s, ids, n);
-  if (copied) p.receivers = s->d_copy_receivers.as<DevReceiver>();
+  const bool spread = out == 0 && shape_for(s->exact, s->shape, out) == 0 && rays >= kSpreadRays &&
+                      spread_images(s, ids, n);
+  if (spread) {
+    p.image_step = qm::kImageSpread;
+    p.receivers += s->receivers.size();
+    cuda_check(qm::launch_spread(s->spread, stream), "image spread");
+  }
   cuda_check(launch_trace_mode(s->exact, p, out, stream, s->shape, chunk_iters, work,
-                               copied ? s->copied : qm::CopiedImages()),
+                               spread ? s->spread : qm::SpreadImages()),
              "trace kernel");
   return total;
 }

@@ -51,9 +51,6 @@ struct DevReceiver {
   float3 a, ab, ac;     // rectangle: vertex 0, v1 - v0, v3 - v0
   float3 pos, size;     // cylinder: centre, (radius, height, -)
   float rcp_height;     // cylinder: 1 / height rounded to nearest (host division)
-  // Flux launches: block b deposits into copy (b & copy_mask) of the image,
-  // copy_stride floats apart (0, 0: the image alone).
-  int copy_mask, copy_stride;
 };
 
 // One heliostat to trace (a HeliostatArgument plus the per-heliostat
@@ -115,6 +112,8 @@ constexpr int kChunk = 32 * kChunkIters;
 // (qrt::chunk_iters_for): a chunk's iterations run one after another.
 constexpr int kSmallChunkIters = 8;
 constexpr int kMediumChunkIters = 16;
+// Floats from one pixel to the next of a spread image (SpreadImage in power.h).
+constexpr int kImageSpread = 9;
 
 #if defined(__CUDACC__)
 // Kernels launched with launch_overlapped begin with this: their blocks may be
@@ -153,6 +152,7 @@ struct TraceParams {
   const DevTask* tasks;
   const long long* facet_prefix;  // num_tasks + 1 prefix sums of warp chunks per task
   int num_tasks;
+  int image_step;                 // flux launches: kImageSpread when the receivers' images are spread ones (else 0)
   long long total_facets;         // end of the launch's warp chunks (chunks [chunk_begin, total_facets))
   long long chunk_begin;          // first warp chunk of the launch (0: all)
   int light_begin, light_end;     // light indexes traced per facet

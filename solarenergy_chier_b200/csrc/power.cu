@@ -33,36 +33,48 @@ __device__ __forceinline__ void merge(double& s, double& c, double s2, double c2
   s = sum;
 }
 
-// Pixels of the copied images, one per thread of the launch's later blocks.
-// Every value is taken and zeroed by one exchange, so a deposit that another
-// stream's launch makes meanwhile is counted here or by its own merge.
-__device__ __forceinline__ void merge_copies(const CopiedImages& images, long long i) {
+// Pixel i of the spread images, moved into the spread image or (kBack) back.
+// The value is taken and zeroed by one exchange, so a deposit that another
+// stream's launch makes meanwhile is counted here or by its own move back.
+template <bool kBack>
+__device__ __forceinline__ void move_pixel(const SpreadImages& images, long long i) {
   for (int r = 0; r < images.n; ++r) {
-    const CopiedImage& m = images.at[r];
+    const SpreadImage& m = images.at[r];
     if (i >= m.pixels) {
       i -= m.pixels;
       continue;
     }
-    float s = 0.0f;
-#pragma unroll 8
-    for (int k = 0; k < m.copies_n; ++k) s += atomicExch(m.copies + (size_t)k * m.stride + i, 0.0f);
-    if (s != 0.0f) atomicAdd(m.image + i, s);
+    float *flat = m.image + i, *wide = m.spread + i * m.step;
+    const float v = atomicExch(kBack ? wide : flat, 0.0f);
+    if (v != 0.0f) atomicAdd(kBack ? flat : wide, v);
     return;
   }
+}
+
+__global__ void __launch_bounds__(256) spread_kernel(SpreadImages images) {
+  wait_previous();
+  begin_next();
+  move_pixel<false>(images, (long long)blockIdx.x * blockDim.x + threadIdx.x);
+}
+
+long long pixels_of(const SpreadImages& images) {
+  long long pixels = 0;
+  for (int r = 0; r < images.n; ++r) pixels += images.at[r].pixels;
+  return pixels;
 }
 
 // A task's partials are a chain of loads and dependent adds per lane, so the
 // kernel's time is its longest chain: 8 or 32 warps shorten it for tasks of
 // many chunks, where a warp alone would take hundreds of steps.  Blocks from
-// power_blocks on merge the copied images, in the same launch.
+// power_blocks on move the spread images back, in the same launch.
 template <int kWarps>
 __global__ void __launch_bounds__(kWarps > 4 ? 32 * kWarps : 128)
-    power_reduce_kernel(TraceParams p, CopiedImages images, int power_blocks) {
+    power_reduce_kernel(TraceParams p, SpreadImages images, int power_blocks) {
   __shared__ double part[kWarps][2];
   wait_previous();
   begin_next();
   if ((int)blockIdx.x >= power_blocks) {
-    merge_copies(images, (long long)(blockIdx.x - power_blocks) * blockDim.x + threadIdx.x);
+    move_pixel<true>(images, (long long)(blockIdx.x - power_blocks) * blockDim.x + threadIdx.x);
     return;
   }
   const int lane = threadIdx.x & 31, warp = kWarps > 1 ? threadIdx.x >> 5 : 0;
@@ -103,10 +115,13 @@ __global__ void __launch_bounds__(kWarps > 4 ? 32 * kWarps : 128)
 
 }  // namespace
 
-cudaError_t launch_trace_end(const TraceParams& p, const CopiedImages& images, cudaStream_t stream) {
+cudaError_t launch_spread(const SpreadImages& images, cudaStream_t stream) {
+  return launch_overlapped(spread_kernel, (unsigned)((pixels_of(images) + 255) / 256), 256, stream, images);
+}
+
+cudaError_t launch_trace_end(const TraceParams& p, const SpreadImages& images, cudaStream_t stream) {
   const bool power = p.chunk_power && p.num_tasks > 0;
-  long long pixels = 0;
-  for (int r = 0; r < images.n; ++r) pixels += images.at[r].pixels;
+  const long long pixels = pixels_of(images);
   if (!power && pixels == 0) return cudaSuccess;
   // 8 warps per task from 256 chunks a task on (one step per lane), 32 from
   // 1,024: a lone heliostat of 6,400 chunks takes 7 steps of 32 warps, where 8

@@ -8,18 +8,19 @@
 #include "device_scene.h"
 
 namespace qm {
-// Images deposited through copies (DevReceiver::copy_mask): each copy's pixels
-// are added to the image and left zero.
-struct CopiedImage {
+// An image deposited through a spread one, where pixel i is at i * step.
+struct SpreadImage {
   float* image;
-  float* copies;  // `copies_n` of them, `stride` floats apart
-  int pixels, copies_n, stride;
+  float* spread;
+  int pixels, step;
 };
-constexpr int kMaxCopiedImages = 4;
-struct CopiedImages {
+constexpr int kMaxSpreadImages = 4;
+struct SpreadImages {
   int n = 0;
-  CopiedImage at[kMaxCopiedImages];
+  SpreadImage at[kMaxSpreadImages];
 };
-// The end of a trace launch: the power sums, and the copied images' merge.
-cudaError_t launch_trace_end(const TraceParams& p, const CopiedImages& images, cudaStream_t stream);
+// Moves the images into their spread ones.
+cudaError_t launch_spread(const SpreadImages& images, cudaStream_t stream);
+// The end of a trace launch: the power sums, and the spread images' move back.
+cudaError_t launch_trace_end(const TraceParams& p, const SpreadImages& images, cudaStream_t stream);
 }  // namespace qm

@@ -148,11 +148,10 @@ struct qmcrt_scene {
   qrt::DBuf d_power, d_diag;
   qrt::DBuf d_chunk_power;  // per-chunk FP64 power partials of a launch (grows to the largest launch)
   qrt::DBuf d_work;         // work counter of persistent flux launches
-  // Image copies of flux launches onto small receivers (zero between
-  // launches), and the receiver table whose images they are.
-  qrt::DBuf d_copies, d_copy_receivers;
-  qm::CopiedImages copied;
-  bool copies_ready = false;
+  // Spread images of flux launches onto small receivers (zero between
+  // launches); d_receivers holds the receivers a second time with these.
+  qrt::DBuf d_spread;
+  qm::SpreadImages spread;
   // One task per heliostat.  The host copy holds what does not depend on the
   // sun; the normals, frames and walk codes are the device copy's alone,
   // prepared there for every new sun from d_items and d_sun.
@@ -208,8 +207,7 @@ struct qmcrt_scene {
     d_power.release();
     d_chunk_power.release();
     d_work.release();
-    d_copies.release();
-    d_copy_receivers.release();
+    d_spread.release();
     d_diag.release();
     d_tasks.release();
     d_prefix.release();
@@ -234,7 +232,7 @@ qm::SunParams sun_params(float3 sun_dir, float tan_local, float slope_angle);
 // chunk_iters: chunk_iters_for's answer for the launch.
 cudaError_t launch_trace_mode(int mode, const qm::TraceParams& p, int out, cudaStream_t st, int shape, int chunk_iters,
                               unsigned long long* work_counter = nullptr,
-                              const qm::CopiedImages& images = qm::CopiedImages());
+                              const qm::SpreadImages& images = qm::SpreadImages());
 // Warp-chunk iterations of a launch of (mode, shape, out) over `rays` rays; a
 // chunk holds 32 rays per iteration.
 int chunk_iters_for(int mode, int shape, int out, long long rays);

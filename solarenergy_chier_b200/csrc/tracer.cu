@@ -407,7 +407,7 @@ struct FacetWindow {
   // g in [0, P) plus a light index in [0, L) needs no wrap-around).
   const float4* samples[kThreads / 32];
   const float4* perturbations[kThreads / 32];
-  float* image[kThreads / 32];     // where the warp's flux goes (DevReceiver::copy_mask)
+  float* image[kThreads / 32];     // the task's receiver's image
   int shadow_free[kThreads / 32];  // the task's shadow-walk code (DevTask::shadow_free)
   float4 o[kThreads];   // origin.xyz, pool offset g[f] (int bits)
   float4 u[kThreads];   // frame u.xyz, pool offset g[(f+1) % P] (int bits; bit 31: block walk skippable)
@@ -487,7 +487,8 @@ __device__ __forceinline__ void splat_column(const DevReceiver& R, float X, floa
 #endif
 
 // kIters: warp-chunk iterations (kChunkIters, fewer in small flux launches).
-template <int kOut, int kIters = kChunkIters>
+// kStep: floats from one pixel to the next of the receivers' images.
+template <int kOut, int kIters = kChunkIters, int kStep = 1>
 #ifndef QM_TRACE_MIN_BLOCKS
 #define QM_TRACE_MIN_BLOCKS 4
 #endif
@@ -540,7 +541,7 @@ __global__ void __launch_bounds__(kThreads, QM_TRACE_MIN_BLOCKS) trace_kernel(QM
   const DevReceiver& R = p.receivers[T.receiver];
   if (lane == 0) {
     win.shadow_free[threadIdx.x >> 5] = T.shadow_free;
-    win.image[threadIdx.x >> 5] = R.image + (size_t)(blockIdx.x & R.copy_mask) * R.copy_stride;
+    win.image[threadIdx.x >> 5] = R.image;
     win.samples[threadIdx.x >> 5] = T.samples;
     win.perturbations[threadIdx.x >> 5] = T.perturbations;
   }
@@ -667,7 +668,7 @@ __global__ void __launch_bounds__(kThreads, QM_TRACE_MIN_BLOCKS) trace_kernel(QM
               ++clamped;
             }
             const int pix = row * R.resolution.x + col;
-            atomicAdd(lds_image(win.image[threadIdx.x >> 5]) + pix, e);
+            atomicAdd(lds_image(win.image[threadIdx.x >> 5]) + (long long)pix * kStep, e);
             power += (double)e;
             code = pix;
             }
@@ -779,6 +780,17 @@ cudaError_t QM_SYM(launch_trace)(const TraceParams& params, int out, cudaStream_
     case kOutBits: trace_kernel<kOutBits><<<(unsigned)blocks, threads, 0, stream>>>(QM_TRACE_LAUNCH_ARGS); break;
     default:
 #if QM_CHUNK_ITERS == 64 && QM_TRACE_THREADS != 64 && !defined(QM_TRACE_PERSISTENT)
+      if (p.image_step == kImageSpread) {
+        switch (chunk_iters) {
+          case kSmallChunkIters:
+            return launch_overlapped(trace_kernel<kOutFlux, kSmallChunkIters, kImageSpread>, (unsigned)blocks, threads, stream, p);
+          case kMediumChunkIters:
+            return launch_overlapped(trace_kernel<kOutFlux, kMediumChunkIters, kImageSpread>, (unsigned)blocks, threads, stream, p);
+          case kChunkIters:
+            return launch_overlapped(trace_kernel<kOutFlux, kChunkIters, kImageSpread>, (unsigned)blocks, threads, stream, p);
+        }
+        return cudaErrorInvalidValue;
+      }
       if (chunk_iters == kSmallChunkIters) {
         return launch_overlapped(trace_kernel<kOutFlux, kSmallChunkIters>, (unsigned)blocks, threads, stream, p);
       }
@@ -786,7 +798,7 @@ cudaError_t QM_SYM(launch_trace)(const TraceParams& params, int out, cudaStream_
         return launch_overlapped(trace_kernel<kOutFlux, kMediumChunkIters>, (unsigned)blocks, threads, stream, p);
       }
 #endif
-      if (chunk_iters != kChunkIters) return cudaErrorInvalidValue;
+      if (chunk_iters != kChunkIters || p.image_step > 1) return cudaErrorInvalidValue;
       trace_kernel<kOutFlux><<<(unsigned)blocks, threads, 0, stream>>>(QM_TRACE_LAUNCH_ARGS);
       break;
   }

@@ -155,12 +155,12 @@ def test_chunk_sizes_of_small_launches(heliostats, lights, tmp_path):
 
 
 @pytest.mark.parametrize("mode", [0, 1])
-def test_image_copies_of_small_receivers(mode, tmp_path):
+def test_spread_images_of_small_receivers(mode, tmp_path):
     """Flux launches of 1.5 M rays and more onto small receivers deposit
-    through copies of the images: one launch gives what smaller launches over
-    the same lights add up to directly (L1 <= 1e-6, FP64 powers 1e-12), on
-    both receivers of a scene, a second launch adds to the images, and
-    nothing is left in the copies."""
+    into spread images: one launch gives what smaller launches over the same
+    lights add up to directly (L1 <= 1e-6, FP64 powers 1e-12), on both
+    receivers of a scene, a second launch adds to the images, and nothing is
+    left in the spread ones."""
     f = synth.two_receiver_field(tmp_path, seed=1, helio_pixel=0.05, groups=4, per_group=128)
     s = q.Scene(f.scene, f.config, device=0, seed=2)
     s.set_math_mode(mode)
