@@ -195,6 +195,8 @@ std::vector<DevReceiver> with_spread_images(qmcrt_scene* s) {
   return recv;
 }
 
+constexpr size_t kFirstChunks = 8192;  // 64 KiB of power partials made with a scene
+
 void build_device_scene(qmcrt_scene* s) {
   qm::SceneModel& m = s->model;
   const qm::SceneConfig& cfg = m.config;
@@ -277,6 +279,10 @@ void build_device_scene(qmcrt_scene* s) {
     s->images.push_back(std::move(img));
   }
   upload(s->d_receivers, with_spread_images(s));
+  // A first small trace then allocates nothing but its chunk table (one
+  // heliostat's first pass 530-610 -> 136 us).
+  s->d_chunk_power.alloc(kFirstChunks * sizeof(double));
+  s->d_work.alloc(sizeof(unsigned long long));
 
   // Focus-flat local facet frames.
   std::vector<float3> local;
