@@ -386,7 +386,9 @@ void update_walk_codes(qmcrt_scene* s) {
 
 // The tracer's copies of the pools (world-space samples, P + L entries);
 // redone after every change of the pools or of the sun, with the walk codes
-// that depend on both.  Returns when the device is done.
+// that depend on both.  Traces of any stream read both: callers wait for the
+// device first (the legacy stream does not wait for non-blocking ones).
+// Returns when the device is done.
 void rotate_pool(qmcrt_scene* s) {
   const int n_out = s->pool_size + s->model.config.num_per_sunshape_group;
   cuda_check(qm::launch_trace_pools(s->d_samples.as<float4>(), s->d_perturb.as<float4>(), s->pool_size, n_out, s->sun,
@@ -432,6 +434,7 @@ void generate_pool(qmcrt_scene* s, unsigned seed, int sunshape, float half_angle
              "pool bound");
   qm::PoolStats found;
   cuda_check(cudaMemcpy(&found, stats, sizeof(found), cudaMemcpyDeviceToHost), "pool kernel");
+  cuda_check(cudaDeviceSynchronize(), "pool kernel");
   set_pool_bounds(s, found);
   rotate_pool(s);
 }
@@ -922,6 +925,7 @@ int qmcrt_set_sample_pool(qmcrt_scene* s, const float* dirs, const float* pertur
     qm::PoolStats found;
     cuda_check(cudaMemcpy(&found, stats, sizeof(found), cudaMemcpyDeviceToHost), "pool check");
     if (found.bad) invalid("sample-pool vectors must be unit vectors (squared length in [0.25, 4])");
+    cuda_check(cudaDeviceSynchronize(), "pool check");
     cuda_check(qm::launch_xyz_to_float4(stage_dirs, s->d_samples.as<float4>(), n, 0), "pool convert");
     cuda_check(qm::launch_xyz_to_float4(stage_pert, s->d_perturb.as<float4>(), n, 0), "pool convert");
     set_pool_bounds(s, found);
