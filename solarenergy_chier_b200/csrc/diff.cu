@@ -323,7 +323,9 @@ __device__ __forceinline__ void ray_adjoint(const ChunkConstants& T, const Facet
   const Dual3T<0> dnp = normalize(slope);
   const Dual3T<0> din3 = d3<0>(make_float3(-din.x, -din.y, -din.z));
   const DualT<0> c0 = dot(dnp, din3);
-  const Dual3T<0> drd = normalize(din3 - dnp * (c0 * 2.0f));
+  const Dual3T<0> refl = din3 - dnp * (c0 * 2.0f);
+  const DualT<0> inv_len = drsqrt(dot(refl, refl));
+  const Dual3T<0> drd = refl * inv_len;  // normalize(refl)
   const float3 d = val(drd), np = val(dnp), in = val(din3);
   float t, u, v;
   // The receiver test with its decisions rounded as the forward's and the
@@ -441,10 +443,12 @@ __device__ __forceinline__ void ray_adjoint(const ChunkConstants& T, const Facet
   }
   add_outer(sum, obar, fd.local);
   if (fd.identity) return;  // the slope-error frame does not turn
-  // rd = in - 2 (np . in) np and c = -(np . in) (np is a unit vector; rd keeps
-  // in's length, so its normalisation has no derivative), then np = slope / |slope|.
+  // rd = (in - 2 (np . in) np) / |in| and c = -(np . in) / |in| (np is a unit
+  // vector, so the reflection keeps in's length, which no parameter moves but
+  // which is not always 1: pools and suns need not be of unit length), then
+  // np = slope / |slope|.
   const float rn = qm::dot(rdbar, np);
-  const float3 npbar = axpy(-2.0f * rn - cbar, in, qm::mul(rdbar, -2.0f * c0.v));
+  const float3 npbar = qm::mul(axpy(-2.0f * rn - cbar, in, qm::mul(rdbar, -2.0f * c0.v)), inv_len.v);
   const float il = rsqrtf(dot(slope, slope).v);
   const float3 wbar = qm::mul(axpy(-qm::dot(npbar, np), np, npbar), il);
   // slope = pert.x u + pert.y n + pert.z v with, for n = (s sin psi, n.y,
