@@ -48,13 +48,13 @@ __device__ __forceinline__ DualT<N> dc(float v) {
   DualT<N> r;
   r.v = v;
 #pragma unroll
-  for (int k = 0; k < N; ++k) r.d[k] = 0.0f;
+  for (int k = 0; k < N; ++k) r.d[k] = 0.0;
   return r;
 }
 template <int N>
 __device__ __forceinline__ DualT<N> dvar(float v, int k) {
   DualT<N> r = dc<N>(v);
-  r.d[k] = 1.0f;
+  r.d[k] = 1.0;
   return r;
 }
 template <int N>
@@ -104,7 +104,7 @@ __device__ __forceinline__ DualT<N> drsqrt(DualT<N> a) {
   DualT<N> o;
   o.v = r;
   if constexpr (N > 0) {
-    const float dr = -0.5f * r * r * r;
+    const double dr = -0.5 / ((double)a.v * sqrt((double)a.v));
 #pragma unroll
     for (int k = 0; k < N; ++k) o.d[k] = dr * a.d[k];
   }
@@ -294,6 +294,10 @@ __device__ __forceinline__ void add_outer(FrameSum& s, float3 a, float3 l) {
   s.n.x += a.x * l.y; s.n.y += a.y * l.y; s.n.z += a.z * l.y;
   s.v.x += a.x * l.z; s.v.y += a.y * l.z; s.v.z += a.z * l.z;
 }
+// abar . da/d(parameter k)
+__device__ __forceinline__ double along(float3 abar, const Dual3T<K>& a, int k) {
+  return abar.x * a.x.d[k] + abar.y * a.y.d[k] + abar.z * a.z.d[k];
+}
 __device__ __forceinline__ float3 axpy(float s, float3 x, float3 y) {
   return make_float3(s * x.x + y.x, s * x.y + y.y, s * x.z + y.z);
 }
@@ -305,6 +309,7 @@ struct ChunkConstants {
   const float4* samples;
   const float4* perturbations;
   float factor;
+  float sx, sy;  // cylinder: pixels per radian, per metre of height
 };
 
 // Adds the contribution of one ray (facet fd, light lab) that hit the
@@ -424,8 +429,8 @@ __device__ __forceinline__ void ray_adjoint(const ChunkConstants& T, const Facet
     float3 qbar, m;
     float md;
     if (R.type == 1) {
-      const float a = __fdividef(xbar * ((float)R.resolution.x * (1.0f / kTwoPi)), rr);
-      qbar = make_float3(-a * z, ybar * ((float)R.resolution.y * R.rcp_height), a * x);
+      const float a = __fdividef(xbar * T.sx, rr);
+      qbar = make_float3(-a * z, ybar * T.sy, a * x);
       m = make_float3(x, 0.0f, z);
       md = den;
     } else {
@@ -489,15 +494,17 @@ __device__ __forceinline__ float3 get3(const AdjointWindow& w, int first, int sl
   return make_float3(w.value[first][slot], w.value[first + 1][slot], w.value[first + 2][slot]);
 }
 
-// Bound by instruction issue (76 % of the slots; 15.5 warp instructions a ray
-// at 8 lights per facet, 13.4 at 32).  Run backwards a ray costs its value chain, one
+// Bound by instruction issue.  Run backwards a ray costs its value chain, one
 // sweep of vector adjoints and 18 multiply-adds into the frame sums, against
-// four tangents through every operation (34 warp instructions a ray); the
-// queue gives every sweep 32 hits where a chunk's iterations hold 22 on the
-// benchmark field.  462 M rays, 32 lights per facet: 17.9 -> 7.4 ms (11.7 of it
-// before the shared constants and the four-pixel read, 7.8 before the sweep
-// stood in the code once and the facets apart from it: 15 % of the stalls
-// waited for instructions); 256 M rays, 4 lights: 11.9 -> 5.5, 6.6 before that.
+// four tangents through every operation; the queue gives every sweep 32 hits
+// where a chunk's iterations hold 22 on the benchmark field.  The call on 462 M
+// rays, 32 lights per facet: 17.9 -> 7.7 ms; on 256 M rays, 4 lights: 11.9 -> 5.8.
+// Distance (2-norm) from 64-bit tangents of the same rays, over four fields x 16
+// seeds: 3.3e-8 to 4.6e-8, where the forward-mode kernel's was 3.6e-8 to 8.1e-8:
+// what counts is the factors that a heliostat's rays share (its tangents, the
+// pixels per radian), hence in double; the sweep's three approximate divisions
+// round each ray on its own, and IEEE ones (0.3 ms more) leave the distance at
+// 3.4e-8 to 4.4e-8.
 // 20 / 24 / 28 blocks per SM: 8.2 / 7.9 / 8.3 ms with the facets still inlined.
 __global__ void __launch_bounds__(kBwdThreads, QM_BWD_MIN_BLOCKS) diff_backward_kernel(BackwardParams p) {
   __shared__ AdjointWindow win;
@@ -517,6 +524,8 @@ __global__ void __launch_bounds__(kBwdThreads, QM_BWD_MIN_BLOCKS) diff_backward_
     c.samples = T.samples;
     c.perturbations = T.perturbations;
     c.factor = T.factor;
+    c.sx = (float)(c.R.resolution.x / 6.283185307179586);
+    c.sy = (float)c.R.resolution.y / c.R.size.y;
   }
   const int r_end = T.num_facets * nl;
   const int iters = min(kChunkIters, (r_end - r0 + 31) >> 5);
@@ -599,10 +608,7 @@ __global__ void __launch_bounds__(kBwdThreads, QM_BWD_MIN_BLOCKS) diff_backward_
   if (DT.identity) return;
 #pragma unroll
   for (int k = 0; k < K; ++k) {
-    const float3 du = make_float3(DT.u.x.d[k], DT.u.y.d[k], DT.u.z.d[k]);
-    const float3 dn = make_float3(DT.fn.x.d[k], DT.fn.y.d[k], DT.fn.z.d[k]);
-    const float3 dv = make_float3(DT.v.x.d[k], DT.v.y.d[k], DT.v.z.d[k]);
-    double s = qm::dot(sum.u, du) + qm::dot(sum.n, dn) + qm::dot(sum.v, dv);
+    double s = along(sum.u, DT.u, k) + along(sum.n, DT.fn, k) + along(sum.v, DT.v, k);
     for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
     if (lane == 0 && s != 0.0) atomicAdd(p.grad + (size_t)T.power_slot * K + k, s);
   }

@@ -12,11 +12,13 @@ namespace qm {
 constexpr int kDiffParams = 4;  // per heliostat: aim offset u, v (m); normal offset u, v (rad)
 
 // A float and its derivatives with respect to N parameters (0: the value
-// alone, by the same operations).
+// alone, by the same operations).  The derivatives are those of one heliostat
+// and scale its whole gradient: in double, so that they add no rounding of
+// their own.
 template <int N>
 struct DualT {
   float v;
-  float d[N > 0 ? N : 1];
+  double d[N > 0 ? N : 1];
 };
 template <int N>
 struct Dual3T {
