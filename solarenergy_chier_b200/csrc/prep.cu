@@ -66,9 +66,12 @@ __global__ void prep_kernel(PrepInputs p) {
   int2 rc;
   heliostat_record(v, it.num_sub, T.row_col, T.pos, normal, it.bound, &rc);
   *it.hsub = make_int4(it.sub_first, it.num_sub, rc.x, rc.y);
+  // A box without a finite top (a heliostat whose aim lies exactly along the
+  // sun's direction has no normal) must not lower the height at which the walks
+  // of the others end: the NaN's key is the largest of all.
   const float4 *c = it.bound;
-  atomicMax(it.top_key, height_key(__float_as_int(c[0].y + fabsf(c[1].y) * c[1].w + fabsf(c[2].y) * c[2].w +
-                                                  fabsf(c[3].y) * c[3].w)));
+  const float top = c[0].y + fabsf(c[1].y) * c[1].w + fabsf(c[2].y) * c[2].w + fabsf(c[3].y) * c[3].w;
+  atomicMax(it.top_key, height_key(isfinite(top) ? __float_as_int(top) : 0x7f800000));
 }
 
 // DevGrid::sub_free code of a block_candidates result: 1 nothing to hit,

@@ -410,6 +410,37 @@ def test_walks_that_end_above_the_mirrors(elevation, tmp_path):
     assert blocked > 0
 
 
+def test_a_heliostat_without_a_normal_leaves_the_others_alone(tmp_path):
+    """A sun that travels exactly along one heliostat's direction to its aim
+    point gives that heliostat a NaN normal and a NaN box.  The others, which
+    walk past it in the dense field, keep their shadowing and blocking: per-ray
+    outcomes of the exact build identical to the oracle's."""
+    import json
+    from pathlib import Path
+
+    f = synth.huge_field(tmp_path, seed=5, helio_pixel=1.0, receiver_pixel=0.2, groups=4, per_group=128)
+    s = q.Scene(f.scene, f.config, device=0, seed=3)
+    s.set_sun([0.0, -1e-30, 0.0])  # too short to turn a normal: it is the direction to the aim point
+    sun = s.heliostat(0)["normal"]
+    s.set_sun(sun)
+    assert np.isnan(s.heliostat(0)["normal"]).all() and not np.isnan(s.heliostat(1)["normal"]).any()
+    cfg = json.loads(Path(f.config).read_text())
+    Path(f.config).write_text(json.dumps(dict(cfg, sun_dir=[float(x) for x in sun])))
+    s.generate_sample_pool(7)
+    dirs, pert = s.get_sample_pool()
+    o = oracle.OracleScene.from_files(f.scene, f.config)
+    s.set_math_mode(1)
+    blocked = 0
+    for h in range(1000, 10000, 1000):
+        offsets = {h: s.get_facet_offsets(h)}
+        nf, L = s.heliostat(h)["num_facets"], s.lights_per_group
+        want = o.trace([h], dirs, pert, offsets, record=(h, 0, nf), images=False)["records"]
+        got = s.hit_records(h, 0, nf, 0, L)
+        assert np.array_equal(got, want), f"heliostat {h}: {np.mean(got != want):.2e} differ"
+        blocked += int(np.sum(want == -2))
+    assert blocked > 0
+
+
 def test_sharded_trace_one_rank_equals_plain(small):
     """shard.ShardedTrace over a one-rank NCCL group: the collectives run on
     the tracer's own device image (a zero-copy view) and give the plain trace."""
