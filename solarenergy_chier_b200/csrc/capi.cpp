@@ -13,6 +13,7 @@
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
+#include <limits>
 #include <memory>
 #include <stdexcept>
 #include <string>
@@ -279,8 +280,11 @@ void build_device_scene(qmcrt_scene* s) {
     s->images.push_back(std::move(img));
   }
   upload(s->d_receivers, with_spread_images(s));
-  // A first small trace then allocates nothing but its chunk table (one
-  // heliostat's first pass 530-610 -> 136 us).
+  // The chunk prefix of a list of one task: kernels take a task's end as the
+  // launch's when that comes first.
+  upload(s->d_single, std::vector<long long>{0, std::numeric_limits<long long>::max()});
+  // A first small trace then allocates nothing (one heliostat's first pass
+  // 530-610 -> 136 us).
   s->d_chunk_power.alloc(kFirstChunks * sizeof(double));
   s->d_work.alloc(sizeof(unsigned long long));
 
@@ -600,21 +604,12 @@ long long trace_ids(qmcrt_scene* s, const int* ids, int n, cudaStream_t stream, 
   for (int i = 0; i < n; ++i) total += chunks_of(ids[i]);
   qm::TraceParams p = base_params(s);
   if (n == 1) {
-    // One heliostat, as the reference traces them: its task and its chunk
-    // count lie on the device, so a call uploads nothing.
-    if (s->single_lights != nl || s->single_chunk != chunk) {
-      std::vector<long long> single(2 * s->templates.size(), 0);
-      for (size_t h = 0; h < s->templates.size(); ++h) single[2 * h + 1] = chunks_of((int)h);
-      s->single_lights = -1;
-      s->d_single.alloc(single.size() * sizeof(long long));
-      cuda_check(cudaMemcpyAsync(s->d_single.p, single.data(), single.size() * sizeof(long long), cudaMemcpyHostToDevice,
-                                 stream),
-                 "chunk table");
-      s->single_lights = nl;
-      s->single_chunk = chunk;
-    }
+    // One heliostat, as the reference traces them: its task lies on the
+    // device and its chunks are the launch's, so a call uploads nothing and
+    // keeps nothing that another light range, stream or captured graph could
+    // find changed.
     p.tasks = s->d_templates.as<DevTask>() + ids[0];
-    p.facet_prefix = s->d_single.as<long long>() + 2 * (size_t)ids[0];
+    p.facet_prefix = s->d_single.as<long long>();
   } else {
     const bool listed = (int)s->cached_ids.size() == n && std::equal(ids, ids + n, s->cached_ids.begin());
     if (!listed || s->cached_lights != nl || s->cached_chunk != chunk) {

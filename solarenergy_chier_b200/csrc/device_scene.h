@@ -150,7 +150,7 @@ struct TraceParams {
   const DevGrid* grids;
   const DevReceiver* receivers;
   const DevTask* tasks;
-  const long long* facet_prefix;  // num_tasks + 1 prefix sums of warp chunks per task
+  const long long* facet_prefix;  // num_tasks + 1 prefix sums of warp chunks per task (the last may exceed the end)
   int num_tasks;
   int image_step;                 // flux launches: kImageSpread when the receivers' images are spread ones (else 0)
   long long total_facets;         // end of the launch's warp chunks (chunks [chunk_begin, total_facets))

@@ -161,12 +161,12 @@ struct qmcrt_scene {
   mutable bool model_stale = false;  // the model's normals and vertices are an earlier sun's
   // Traced lists: consecutive heliostats are traced from d_templates itself,
   // others from a copy in list order (d_tasks, of the sun it was gathered for).
-  qrt::DBuf d_tasks, d_ids, d_prefix, d_single;
+  qrt::DBuf d_tasks, d_ids, d_prefix;
+  qrt::DBuf d_single;  // chunk prefix of every list of one heliostat
   std::vector<int> cached_ids;
   long long cached_lights = -1;
   long long cached_chunk = -1;
   bool gathered = false;
-  long long single_lights = -1, single_chunk = -1;  // d_single: chunks of each heliostat traced alone
   int shape = 0;  // launch shape of the production build (qmcrt_set_launch_shape)
   int* h_ids = nullptr;  // pinned staging of list uploads
   long long* h_prefix = nullptr;

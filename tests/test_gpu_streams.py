@@ -51,3 +51,60 @@ def test_a_change_waits_for_traces_of_other_streams(change, small):
     torch.cuda.synchronize()
     assert_same(s.image(0), want)
     np.testing.assert_allclose(s.power()[0], power, rtol=1e-9, atol=0)
+
+
+def test_a_captured_call_of_one_heliostat(small):
+    """One-heliostat traces captured right after the light range changed, then
+    replayed after traces of other ranges and lists: the graph depends on no
+    memory of the capturing call."""
+    import torch
+
+    s = q.Scene(small.scene, small.config, device=0, seed=2)
+    s.trace([3])  # another light range before
+    s.set_light_range(5, 42)
+    s.clear()
+    s.trace([3])
+    s.trace([7])
+    want, power = s.image(0), s.power()[0]
+    s.set_light_range(0, 200)
+    s.trace([3])
+    s.set_light_range(5, 42)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        stream = torch.cuda.current_stream()
+        s.trace([3], stream=stream)
+        s.trace([7], stream=stream)
+    s.set_light_range(0, 300)
+    s.trace([9])
+    s.trace([1, 4, 6])
+    for _ in range(2):
+        s.clear()
+        s.clear_power()
+        torch.cuda.synchronize()
+        graph.replay()
+        torch.cuda.synchronize()
+        assert_same(s.image(0), want)
+    assert s.power()[0][7] == pytest.approx(power[7], rel=1e-12)
+
+
+def test_calls_of_one_heliostat_on_several_streams(small):
+    """Calls of different light counts and chunk sizes follow one another on
+    three streams without waiting: the image is that of the calls in turn."""
+    import torch
+
+    s = q.Scene(small.scene, small.config, device=0, seed=2)
+    calls = [(h, lights) for h in range(12) for lights in (16, 2048, 600)]  # 8-, 16- and 8-iteration chunks
+    s.trace(list(range(s.num_heliostats)))  # the power partials' buffer is large enough from here on
+
+    def traced(streams):
+        s.clear()
+        torch.cuda.synchronize()
+        for k, (h, lights) in enumerate(calls):
+            s.set_light_range(0, lights)
+            s.trace([h], stream=streams[k % len(streams)])
+        torch.cuda.synchronize()
+        return s.image(0)
+
+    want = traced([torch.cuda.current_stream()])
+    assert_same(traced([torch.cuda.Stream() for _ in range(3)]), want)
