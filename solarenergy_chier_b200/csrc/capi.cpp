@@ -57,6 +57,12 @@ using qm::DevGrid;
 using qm::DevReceiver;
 using qm::DevTask;
 
+// Waits for the device, after which no launch of the scene is pending.
+void synchronise(qmcrt_scene* s, const char* what) {
+  cuda_check(cudaDeviceSynchronize(), what);
+  s->spread_stream = -1;
+}
+
 qm::SunFrame sun_frame(float3 sun_dir) {
   // -sun_dir (QuasiMonteCarloRayTracer::generateSunrayArgument feeds
   // -sunray_direction to local2world_rotate per ray; the frame is constant).
@@ -161,37 +167,34 @@ void model_for_sun(const qmcrt_scene* s) {
   s->model_stale = false;
 }
 
-// The largest image that has a spread one (see kSpreadRays), 4.5 MiB of it.
-constexpr long long kSpreadPixels = 1 << 17;
+// The largest image that has a spread one (see kSpreadRays), 1.4 MiB of it.
+constexpr long long kSpreadPixels = 40000;
 bool spread_pixels(const DevReceiver& r) { return (long long)r.resolution.x * r.resolution.y <= kSpreadPixels; }
 
 // The scene's receivers, and a second time with the spread images that are
 // made here for the small ones.
 std::vector<DevReceiver> with_spread_images(qmcrt_scene* s) {
   std::vector<DevReceiver> recv = s->receivers;
-  s->spread.n = 0;
+  s->spread.assign(s->receivers.size(), qm::SpreadImage());
   s->d_spread.release();
-  if (recv.size() <= (size_t)qm::kMaxSpreadImages) {
-    size_t floats = 0;
-    for (auto& r : s->receivers) {
-      if (spread_pixels(r)) {
-        const int pixels = r.resolution.x * r.resolution.y;
-        s->spread.at[s->spread.n++] = {r.image, nullptr, pixels, qm::kImageSpread};
-        floats += (size_t)pixels * qm::kImageSpread;
-      }
-      recv.push_back(r);
+  if (s->receivers.size() > (size_t)qm::kMaxSpreadImages) return recv;
+  size_t floats = 0;
+  for (auto& r : s->receivers)
+    if (spread_pixels(r)) floats += (size_t)r.resolution.x * r.resolution.y * qm::kImageSpread;
+  if (floats) {
+    s->d_spread.alloc(floats * sizeof(float));
+    cuda_check(cudaMemset(s->d_spread.p, 0, s->d_spread.bytes), "cudaMemset");
+  }
+  float* next = s->d_spread.as<float>();
+  for (size_t k = 0; k < s->receivers.size(); ++k) {
+    DevReceiver r = s->receivers[k];
+    if (spread_pixels(r)) {
+      const int pixels = r.resolution.x * r.resolution.y;
+      s->spread[k] = {r.image, next, pixels, qm::kImageSpread};
+      r.image = next;
+      next += (size_t)pixels * qm::kImageSpread;
     }
-    if (floats) {
-      s->d_spread.alloc(floats * sizeof(float));
-      cuda_check(cudaMemset(s->d_spread.p, 0, s->d_spread.bytes), "cudaMemset");
-    }
-    float* next = s->d_spread.as<float>();
-    int k = 0;
-    for (size_t r = s->receivers.size(); r < recv.size(); ++r) {
-      if (!spread_pixels(recv[r])) continue;
-      s->spread.at[k++].spread = recv[r].image = next;
-      next += (size_t)recv[r].resolution.x * recv[r].resolution.y * qm::kImageSpread;
-    }
+    recv.push_back(r);
   }
   return recv;
 }
@@ -335,7 +338,7 @@ void generate_offsets(qmcrt_scene* s, unsigned seed) {
   cuda_check(qm::launch_offsets_all(s->d_offsets.as<int>(), s->d_offset_seg.as<long long>(),
                                     (int)s->model.heliostats.size(), total, seed, s->pool_size, 0),
              "offsets kernel");
-  cuda_check(cudaDeviceSynchronize(), "offsets kernel");
+  synchronise(s, "offsets kernel");
 }
 
 // Sun axis and tangent of the largest sun-shape angle in world space, from
@@ -399,7 +402,7 @@ void rotate_pool(qmcrt_scene* s) {
                                     s->d_trace_samples.as<float4>(), s->d_trace_perturb.as<float4>(), 0),
              "pool rotation");
   update_walk_codes(s);
-  cuda_check(cudaDeviceSynchronize(), "pool rotation");
+  synchronise(s, "pool rotation");
 }
 
 void generate_pool(qmcrt_scene* s, unsigned seed, int sunshape, float half_angle) {
@@ -438,7 +441,7 @@ void generate_pool(qmcrt_scene* s, unsigned seed, int sunshape, float half_angle
              "pool bound");
   qm::PoolStats found;
   cuda_check(cudaMemcpy(&found, stats, sizeof(found), cudaMemcpyDeviceToHost), "pool kernel");
-  cuda_check(cudaDeviceSynchronize(), "pool kernel");
+  synchronise(s, "pool kernel");
   set_pool_bounds(s, found);
   rotate_pool(s);
 }
@@ -556,26 +559,52 @@ double* chunk_power_buffer(DBuf& buf, long long chunks) {
 // Deposits onto a small image crowd into few sectors of L2, whose slices then
 // bound the launch (on 160 x 120 pixels the busiest slice's atomic unit was
 // 68 % busy, the average 15 %).  Such launches deposit into a spread image,
-// one pixel per kImageSpread floats, into which a first launch moves the
-// image's values and from which the launch that sums the power moves them
-// back: still one float accumulator per pixel, so a pixel's rounding error
-// is what it was (8 copies of the image, merged, were 0.07 ms faster on 655 M
-// rays but 5e-5 from the sums of one accumulator).  655 M rays of 50
-// heliostats, ms at 1 / 2 / 4 / 6 / 8 / 9 / 12 / 16 / 32 floats a pixel:
-// 8.7 / 7.2 / 7.0 / 6.8 / 7.2 / 6.7 / 7.0 / 7.5 / 8.3: of the steps of a
-// sector and more the odd one does best.  Whole launches, us without / with: one heliostat, 0.4 M rays
-// 14 / 18, 1.6 M 34 / 30, 6.6 M 115 / 84; 50 of them, 1.3 M 32 / 33, 5.1 M
-// 79 / 73, 41 M 548 / 456, 164 M 2,172 / 1,679; hence from 1.5 M rays on.  On the
-// 754,200 pixels of the 624-heliostat field the slices share the load (13 and
-// 19 %).
-constexpr long long kSpreadRays = 1500 * 1000;
+// one pixel per kImageSpread floats, which the launch that sums the power adds
+// to the image: still one float accumulator per pixel in a launch, so that a
+// pixel's rounding error is no more than a direct deposit's, and the image
+// itself keeps its values for readers on other streams.  Launches of 1 / 50
+// heliostats of a small plant, us direct / spread:
+//   pixels   0.8 M rays    1.6 M       13 M       1.3 M      41 M        164 M
+//    4,800   20.4 / 16.8  40 / 32   351 / 215   36 / 30   652 / 470  2,603 / 1,790
+//   19,200   21.3 / 16.9  36 / 28   247 / 147   36 / 30   754 / 460  2,993 / 1,699
+//   23,232   16.7 / 17.8  29 / 28   190 / 147   30 / 30   475 / 460  1,848 / 1,700
+//   30,000   16.7 / 18.4  28 / 28   181 / 148   30 / 30   473 / 460  1,817 / 1,700
+//   37,632   16.6 / 18.4  28 / 28   160 / 148   30 / 30   467 / 460  1,791 / 1,700
+//   43,200   16.7 / 18.5  28 / 28   150 / 148   30 / 30   457 / 461  1,691 / 1,701
+//   52,272   16.8 / 18.5  28 / 28   148 / 148   30 / 30   457 / 461  1,691 / 1,700
+//  120,000   16.7 / 19.7  28 / 29   147 / 148   30 / 31   459 / 461  1,696 / 1,701
+// and below 0.7 M rays direct is never slower.  Hence from 1 M rays on, on up to
+// 40,000 pixels.  The step: 655 M rays of 50 heliostats onto 19,200 pixels, ms at
+// 1 / 2 / 4 / 6 / 8 / 9 / 12 / 16 / 32 floats a pixel: 8.7 / 7.2 / 7.0 / 6.8 / 7.2 /
+// 6.7 / 7.0 / 7.5 / 8.3; from a sector on the steps differ little.
+constexpr long long kSpreadRays = 1000 * 1000;
 
-// Whether the receivers of heliostats ids[0..n) all have spread images.
-bool spread_images(const qmcrt_scene* s, const int* ids, int n) {
-  if (s->spread.n == 0) return false;
-  for (int i = 0; i < n; ++i)
-    if (!spread_pixels(s->receivers[s->templates[ids[i]].receiver])) return false;
-  return true;
+// The spread images of the receivers of heliostats ids[0..n), if all have one
+// and a launch on `stream` may use them.  Launches of two streams must not
+// meet in one spread image: the deposits of one would reach the image with
+// the end of the other, after a caller has waited for the first.  So the first
+// stream that spreads keeps the images until the scene has waited for the
+// device (synchronise); launches on others deposit directly, as do captured ones,
+// whose graph may be replayed anywhere.
+qm::SpreadImages spread_images(qmcrt_scene* s, const int* ids, int n, cudaStream_t stream) {
+  qm::SpreadImages images;
+  if (s->spread.size() > (size_t)qm::kMaxSpreadImages) return {};
+  unsigned seen = 0;
+  for (int i = 0; i < n; ++i) {
+    const int r = s->templates[ids[i]].receiver;
+    if (seen >> r & 1u) continue;
+    seen |= 1u << r;
+    if (!s->spread[r].spread) return {};
+    images.at[images.n++] = s->spread[r];
+  }
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  cuda_check(cudaStreamIsCapturing(stream, &capture), "cudaStreamIsCapturing");
+  if (capture != cudaStreamCaptureStatusNone) return {};
+  unsigned long long id = 0;
+  cuda_check(cudaStreamGetId(stream, &id), "cudaStreamGetId");
+  if (s->spread_stream != -1 && s->spread_stream != (long long)id) return {};
+  s->spread_stream = (long long)id;
+  return images;
 }
 
 // Traces heliostats ids[0..n) over the scene's light range: out 0 adds their
@@ -656,16 +685,14 @@ long long trace_ids(qmcrt_scene* s, const int* ids, int n, cudaStream_t stream, 
     if (s->d_work.bytes < sizeof(unsigned long long)) s->d_work.alloc(sizeof(unsigned long long));
     work = s->d_work.as<unsigned long long>();
   }
-  const bool spread = out == 0 && shape_for(s->exact, s->shape, out) == 0 && rays >= kSpreadRays &&
-                      spread_images(s, ids, n);
-  if (spread) {
+  qm::SpreadImages images;
+  if (out == 0 && shape_for(s->exact, s->shape, out) == 0 && rays >= kSpreadRays)
+    images = spread_images(s, ids, n, stream);
+  if (images.n) {
     p.image_step = qm::kImageSpread;
     p.receivers += s->receivers.size();
-    cuda_check(qm::launch_spread(s->spread, stream), "image spread");
   }
-  cuda_check(launch_trace_mode(s->exact, p, out, stream, s->shape, chunk_iters, work,
-                               spread ? s->spread : qm::SpreadImages()),
-             "trace kernel");
+  cuda_check(launch_trace_mode(s->exact, p, out, stream, s->shape, chunk_iters, work, images), "trace kernel");
   return total;
 }
 
@@ -883,7 +910,7 @@ int qmcrt_scene_set_sun(qmcrt_scene* s, const float* sun_dir) {
       return;
     }
     DeviceGuard guard(s->device);
-    cuda_check(cudaDeviceSynchronize(), "set_sun");
+    synchronise(s, "set_sun");
     s->model.config.sun_dir = d;
     s->model_stale = true;
     s->flags_valid = false;
@@ -920,7 +947,7 @@ int qmcrt_set_sample_pool(qmcrt_scene* s, const float* dirs, const float* pertur
     qm::PoolStats found;
     cuda_check(cudaMemcpy(&found, stats, sizeof(found), cudaMemcpyDeviceToHost), "pool check");
     if (found.bad) invalid("sample-pool vectors must be unit vectors (squared length in [0.25, 4])");
-    cuda_check(cudaDeviceSynchronize(), "pool check");
+    synchronise(s, "pool check");
     cuda_check(qm::launch_xyz_to_float4(stage_dirs, s->d_samples.as<float4>(), n, 0), "pool convert");
     cuda_check(qm::launch_xyz_to_float4(stage_pert, s->d_perturb.as<float4>(), n, 0), "pool convert");
     set_pool_bounds(s, found);
@@ -1100,7 +1127,7 @@ int qmcrt_receiver_image(qmcrt_scene* s, int id, float* out, int* width, int* he
     if (height) *height = r.resolution.y;
     if (out) {
       DeviceGuard guard(s->device);
-      cuda_check(cudaDeviceSynchronize(), "synchronise");
+      synchronise(s, "synchronise");
       cuda_check(cudaMemcpy(out, s->images[id]->p, (size_t)r.resolution.x * r.resolution.y * sizeof(float),
                             cudaMemcpyDeviceToHost),
                  "image readback");
@@ -1134,7 +1161,7 @@ int qmcrt_power_fp64(qmcrt_scene* s, double* per, double* total) {
     checked(s);
     DeviceGuard guard(s->device);
     std::vector<double> v(s->model.heliostats.size());
-    cuda_check(cudaDeviceSynchronize(), "synchronise");
+    synchronise(s, "synchronise");
     if (!v.empty())
       cuda_check(cudaMemcpy(v.data(), s->d_power.p, v.size() * sizeof(double), cudaMemcpyDeviceToHost), "readback");
     if (per) std::copy(v.begin(), v.end(), per);
@@ -1155,7 +1182,7 @@ int qmcrt_power_clear(qmcrt_scene* s) {
   return guarded([&] {
     checked(s);
     DeviceGuard guard(s->device);
-    cuda_check(cudaDeviceSynchronize(), "synchronise");
+    synchronise(s, "synchronise");
     cuda_check(cudaMemset(s->d_power.p, 0, s->d_power.bytes), "clear");
     cuda_check(cudaMemset(s->d_diag.p, 0, s->d_diag.bytes), "clear");
   });
@@ -1166,7 +1193,7 @@ int qmcrt_diagnostics(qmcrt_scene* s, unsigned long long* out4) {
     checked(s);
     if (!out4) invalid("output is NULL");
     DeviceGuard guard(s->device);
-    cuda_check(cudaDeviceSynchronize(), "synchronise");
+    synchronise(s, "synchronise");
     cuda_check(cudaMemcpy(out4, s->d_diag.p, qm::kDiagSlots * sizeof(unsigned long long), cudaMemcpyDeviceToHost),
                "readback");
   });
@@ -1250,7 +1277,7 @@ int qmcrt_grid_build_device(qmcrt_scene* s, int grid, float* ms) {
     cudaEventDestroy(e2);
     // The scene's lists are replaced in place (same sizes), so batches that
     // share them keep valid pointers.
-    cuda_check(cudaDeviceSynchronize(), "synchronise");
+    synchronise(s, "synchronise");
     cuda_check(cudaMemcpy(gb.ranges.p, d_ranges.p, (size_t)ncell * sizeof(int2), cudaMemcpyDeviceToDevice),
                "grid ranges");
     if (total > 0)

@@ -33,28 +33,24 @@ __device__ __forceinline__ void merge(double& s, double& c, double s2, double c2
   s = sum;
 }
 
-// Pixel i of the spread images, moved into the spread image or (kBack) back.
-// The value is taken and zeroed by one exchange, so a deposit that another
-// stream's launch makes meanwhile is counted here or by its own move back.
-template <bool kBack>
-__device__ __forceinline__ void move_pixel(const SpreadImages& images, long long i) {
+// Adds pixel i of the spread images to its image, where a caller's other
+// streams may read or deposit at the same time.  A spread image belongs to
+// launches of one stream at a time (see spread_images in capi.cpp).
+__device__ __forceinline__ void add_spread(const SpreadImages& images, long long i) {
   for (int r = 0; r < images.n; ++r) {
     const SpreadImage& m = images.at[r];
     if (i >= m.pixels) {
       i -= m.pixels;
       continue;
     }
-    float *flat = m.image + i, *wide = m.spread + i * m.step;
-    const float v = atomicExch(kBack ? wide : flat, 0.0f);
-    if (v != 0.0f) atomicAdd(kBack ? flat : wide, v);
+    float* wide = m.spread + i * m.step;
+    const float v = __ldcg(wide);
+    if (v != 0.0f) {
+      *wide = 0.0f;
+      atomicAdd(m.image + i, v);
+    }
     return;
   }
-}
-
-__global__ void __launch_bounds__(256) spread_kernel(SpreadImages images) {
-  wait_previous();
-  begin_next();
-  move_pixel<false>(images, (long long)blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 long long pixels_of(const SpreadImages& images) {
@@ -66,7 +62,7 @@ long long pixels_of(const SpreadImages& images) {
 // A task's partials are a chain of loads and dependent adds per lane, so the
 // kernel's time is its longest chain: 8 or 32 warps shorten it for tasks of
 // many chunks, where a warp alone would take hundreds of steps.  Blocks from
-// power_blocks on move the spread images back, in the same launch.
+// power_blocks on add the spread images, in the same launch.
 template <int kWarps>
 __global__ void __launch_bounds__(kWarps > 4 ? 32 * kWarps : 128)
     power_reduce_kernel(TraceParams p, SpreadImages images, int power_blocks) {
@@ -74,7 +70,7 @@ __global__ void __launch_bounds__(kWarps > 4 ? 32 * kWarps : 128)
   wait_previous();
   begin_next();
   if ((int)blockIdx.x >= power_blocks) {
-    move_pixel<true>(images, (long long)(blockIdx.x - power_blocks) * blockDim.x + threadIdx.x);
+    add_spread(images, (long long)(blockIdx.x - power_blocks) * blockDim.x + threadIdx.x);
     return;
   }
   const int lane = threadIdx.x & 31, warp = kWarps > 1 ? threadIdx.x >> 5 : 0;
@@ -114,10 +110,6 @@ __global__ void __launch_bounds__(kWarps > 4 ? 32 * kWarps : 128)
 }
 
 }  // namespace
-
-cudaError_t launch_spread(const SpreadImages& images, cudaStream_t stream) {
-  return launch_overlapped(spread_kernel, (unsigned)((pixels_of(images) + 255) / 256), 256, stream, images);
-}
 
 cudaError_t launch_trace_end(const TraceParams& p, const SpreadImages& images, cudaStream_t stream) {
   const bool power = p.chunk_power && p.num_tasks > 0;

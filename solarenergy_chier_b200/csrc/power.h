@@ -8,19 +8,19 @@
 #include "device_scene.h"
 
 namespace qm {
-// An image deposited through a spread one, where pixel i is at i * step.
+// An image deposited through a spread one, where pixel i is at i * step and
+// which holds zeros between launches.
 struct SpreadImage {
-  float* image;
-  float* spread;
-  int pixels, step;
+  float* image = nullptr;
+  float* spread = nullptr;
+  int pixels = 0, step = 0;
 };
 constexpr int kMaxSpreadImages = 4;
 struct SpreadImages {
   int n = 0;
   SpreadImage at[kMaxSpreadImages];
 };
-// Moves the images into their spread ones.
-cudaError_t launch_spread(const SpreadImages& images, cudaStream_t stream);
-// The end of a trace launch: the power sums, and the spread images' move back.
+// The end of a trace launch: the power sums, and the spread images added to
+// theirs.
 cudaError_t launch_trace_end(const TraceParams& p, const SpreadImages& images, cudaStream_t stream);
 }  // namespace qm

@@ -148,10 +148,13 @@ struct qmcrt_scene {
   qrt::DBuf d_power, d_diag;
   qrt::DBuf d_chunk_power;  // per-chunk FP64 power partials of a launch (grows to the largest launch)
   qrt::DBuf d_work;         // work counter of persistent flux launches
-  // Spread images of flux launches onto small receivers (zero between
-  // launches); d_receivers holds the receivers a second time with these.
+  // Spread images of flux launches onto small receivers, one per receiver (none:
+  // spread = NULL); d_receivers holds the receivers a second time with these.
+  // spread_stream: id of the stream whose launches use them, -1 when none of
+  // them can be pending.
   qrt::DBuf d_spread;
-  qm::SpreadImages spread;
+  std::vector<qm::SpreadImage> spread;
+  long long spread_stream = -1;
   // One task per heliostat.  The host copy holds what does not depend on the
   // sun; the normals, frames and walk codes are the device copy's alone,
   // prepared there for every new sun from d_items and d_sun.

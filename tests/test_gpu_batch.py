@@ -184,6 +184,33 @@ def test_spread_images_of_small_receivers(mode, tmp_path):
         np.testing.assert_allclose(p, times * p0, rtol=1e-12, atol=0)
 
 
+@pytest.mark.parametrize("kind,pixel", [("small", 0.0345), ("small", 0.0344), ("two", 0.033)])
+def test_spread_images_and_large_ones(kind, pixel, tmp_path):
+    """Either side of the largest image that has a spread one, and a scene
+    with one receiver on each side: lists of one receiver's heliostats and of
+    both, one launch after another, give what another launch shape's direct
+    deposits do (L1 <= 1e-5, FP64 powers 1e-12)."""
+    make = synth.small_field if kind == "small" else synth.two_receiver_field
+    f = make(tmp_path, seed=1, helio_pixel=0.05, receiver_pixel=pixel, groups=4, per_group=128)
+    s = q.Scene(f.scene, f.config, device=0, seed=2)
+    pixels = [s.receiver(r)["width"] * s.receiver(r)["height"] for r in range(s.num_receivers)]
+    assert [n <= 40000 for n in pixels] == {0.0345: [True], 0.0344: [False], 0.033: [True, False]}[pixel]
+    ids = list(range(s.num_heliostats))
+    half = len(ids) // 2
+    s.set_light_range(0, 24)
+    out = []
+    for shape in (3, 0):  # two-warp blocks never use spread images
+        s.set_launch_shape(shape)
+        s.clear()
+        s.clear_power()
+        for part in (ids, ids[:half], ids[half:], ids[::2]):
+            s.trace(part)
+        out.append(([s.image(r).astype(np.float64) for r in range(s.num_receivers)], s.power()[0]))
+    for a, b in zip(out[1][0], out[0][0]):
+        assert b.sum() > 0 and np.abs(a - b).sum() <= 1e-5 * b.sum()
+    np.testing.assert_allclose(out[1][1], out[0][1], rtol=1e-12, atol=0)
+
+
 def test_every_launch_shape_gives_the_same_result(fields, tmp_path):
     """The autotuner's candidates (launch shapes of the production build:
     block widths, warp chunks of 32, 64 or 128 iterations) change only how

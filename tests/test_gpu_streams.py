@@ -108,3 +108,61 @@ def test_calls_of_one_heliostat_on_several_streams(small):
 
     want = traced([torch.cuda.current_stream()])
     assert_same(traced([torch.cuda.Stream() for _ in range(3)]), want)
+
+
+def test_images_keep_their_values_while_another_stream_traces(small):
+    """Copies of an image taken while another stream traces onto it hold at
+    least what earlier traces left: deposits only add."""
+    import torch
+
+    from solarenergy_chier_b200 import shard
+
+    s = q.Scene(small.scene, small.config, device=0, seed=2)
+    ids = list(range(s.num_heliostats))
+    s.trace(ids)
+    want = torch.from_numpy(s.image(0))
+    view = shard.device_image_tensor(s, 0)
+    tracing, reading = torch.cuda.Stream(), torch.cuda.Stream()
+    copies = [torch.empty_like(want).pin_memory() for _ in range(8)]
+    with torch.cuda.stream(reading):
+        copies[0].copy_(view, non_blocking=True)
+    torch.cuda.synchronize()
+    for _ in range(6):
+        s.trace(ids, stream=tracing)
+    during = 0
+    with torch.cuda.stream(reading):
+        for c in copies:
+            c.copy_(view, non_blocking=True)
+            reading.synchronize()
+            during += not tracing.query()
+    torch.cuda.synchronize()
+    assert during > 0, "no copy was taken during the traces"
+    for c in copies:
+        assert float((want - c).clamp(min=0).sum()) <= 1e-6 * float(want.sum())
+    assert_same(s.image(0), 7.0 * want.numpy())
+
+
+def test_a_waited_trace_is_in_the_image_whatever_other_streams_do(small):
+    """One list traced on two streams: after waiting for one of them alone,
+    the image holds that trace."""
+    import torch
+
+    from solarenergy_chier_b200 import shard
+
+    s = q.Scene(small.scene, small.config, device=0, seed=2)
+    ids = list(range(s.num_heliostats))
+    s.trace(ids)
+    want = torch.from_numpy(s.image(0))
+    view = shard.device_image_tensor(s, 0)
+    got = torch.empty_like(want).pin_memory()
+    a, b = torch.cuda.Stream(), torch.cuda.Stream()
+    for first, second in ((a, b), (b, a), (a, b)):
+        s.clear()
+        torch.cuda.synchronize()
+        s.trace(ids, stream=first)
+        s.trace(ids, stream=second)
+        with torch.cuda.stream(first):
+            got.copy_(view, non_blocking=True)
+            first.synchronize()
+        assert float((want - got).clamp(min=0).sum()) <= 1e-5 * float(want.sum())
+        torch.cuda.synchronize()
