@@ -692,7 +692,10 @@ long long trace_ids(qmcrt_scene* s, const int* ids, int n, cudaStream_t stream, 
     p.image_step = qm::kImageSpread;
     p.receivers += s->receivers.size();
   }
-  cuda_check(launch_trace_mode(s->exact, p, out, stream, s->shape, chunk_iters, work, images), "trace kernel");
+  const cudaError_t e = launch_trace_mode(s->exact, p, out, stream, s->shape, chunk_iters, work, images);
+  // Deposits of a launch whose end was refused must not reach a later one's image.
+  if (e != cudaSuccess && images.n) cudaMemsetAsync(s->d_spread.p, 0, s->d_spread.bytes, stream);
+  cuda_check(e, "trace kernel");
   return total;
 }
 
