@@ -79,7 +79,9 @@ __global__ void __launch_bounds__(kWarps > 4 ? 32 * kWarps : 128)
   const long long c0 = max(__ldg(p.facet_prefix + t), p.chunk_begin);
   const long long c1 = min(__ldg(p.facet_prefix + t + 1), p.total_facets);
   if (c1 <= c0) return;  // the same for all of the task's warps
-  const double* __restrict__ in = p.chunk_power - p.chunk_begin;
+  // Written by the launch that wait_previous waits for: not __restrict__, which
+  // would let the compiler read it as data that no kernel changes, ahead of the wait.
+  const double* in = p.chunk_power - p.chunk_begin;
   constexpr int kStride = 32 * kWarps;
   double s = 0.0, c = 0.0;
   long long k = c0 + (kWarps > 1 ? (int)threadIdx.x : lane);
