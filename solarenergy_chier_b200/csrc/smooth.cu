@@ -256,6 +256,16 @@ namespace {
 // Largest trim that keeps both heaps in registers.
 constexpr int kMaxRegisterTrim = 15;
 
+constexpr size_t kMaxShared = 227 * 1024;  // of a block, and of an SM's blocks together
+
+// Lets a kernel's launches use `smem` bytes of shared memory.  The limit is the
+// kernel's, for all host threads: always the largest one, so that no thread
+// lowers it between another's call here and its launch.
+cudaError_t allow_shared(const void* kernel, size_t smem) {
+  return smem <= 48 * 1024 ? cudaSuccess
+                           : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxShared);
+}
+
 struct RegisterLaunch {
   float* image;      // in place when src is NULL
   const float* src;  // else a copy of the image
@@ -285,18 +295,13 @@ cudaError_t launch_register(int trim, const RegisterLaunch& a) {
   if constexpr (K < kMaxRegisterTrim) {
     if (trim > K) return launch_register<K + 1, kInPlace>(trim, a);
   }
-  constexpr size_t kMaxShared = 227 * 1024;
   const size_t tile_bytes = sizeof(float) * (kTileX + 2 * a.radius) * (kTileY + 2 * a.radius);
   const int tiles_x = (a.width + kTileX - 1) / kTileX;
   const long long tiles = (long long)tiles_x * ((a.height + kTileY - 1) / kTileY);
   if (tiles > INT_MAX) return cudaErrorNotSupported;
   const void* kernel = (const void*)trimmed_mean_register_kernel<K, kInPlace>;
-  auto allow = [&](size_t smem) {
-    return smem <= 48 * 1024 ? cudaSuccess
-                             : cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  };
   if constexpr (!kInPlace) {
-    const cudaError_t e = allow(tile_bytes);
+    const cudaError_t e = allow_shared(kernel, tile_bytes);
     return e != cudaSuccess ? e : start_register<K, false>(a, (int)tiles, tile_bytes, tiles_x, (int)tiles);
   } else {
     int dev = 0, sms = 0, coop = 0, per_sm = 0;
@@ -312,7 +317,7 @@ cudaError_t launch_register(int trim, const RegisterLaunch& a) {
       const long long share = (tiles + (long long)sms * want - 1) / ((long long)sms * want);
       const size_t smem = tile_bytes * share;
       if (smem * want > kMaxShared) continue;
-      e = allow(smem);
+      e = allow_shared(kernel, smem);
       if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, kTileX * kTileY, smem);
       if (e != cudaSuccess) return e;
@@ -350,11 +355,9 @@ cudaError_t launch_trimmed_mean(const float* src, float* dst, int width, int hei
   const dim3 grid((width + block.x - 1) / block.x, (height + block.y - 1) / block.y);
   const int stride = smooth_heap_stride(radius, ratio);
   const size_t smem = sizeof(float) * (size_t)stride * 2 * block.x * block.y;
-  if (smem > 227 * 1024) return cudaErrorInvalidValue;
-  if (smem > 48 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(trimmed_mean_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
+  if (smem > kMaxShared) return cudaErrorInvalidValue;
+  const cudaError_t e = allow_shared((const void*)trimmed_mean_kernel, smem);
+  if (e != cudaSuccess) return e;
   trimmed_mean_kernel<<<grid, block, smem, stream>>>(src, dst, radius, ratio, width, height, stride);
   return cudaGetLastError();
 }

@@ -281,6 +281,44 @@ def test_smoother_tile_and_trim_edges(shape, radius, ratio):
     assert np.array_equal(t.cpu().numpy(), want, equal_nan=True)
 
 
+def test_two_threads_smooth_images_of_different_tiles():
+    """Windows whose tiles need more shared memory than a kernel gets unasked
+    (radius 60 and 64: 76 and 85 KiB), smoothed by two host threads at once:
+    neither lowers the other's limit between its setting and its launch."""
+    import threading
+
+    import torch
+
+    rng = np.random.default_rng(5)
+    img = (rng.random((6, 20)) * 100).astype(np.float32)
+    failures = []
+
+    def work(radius):
+        try:
+            want = oracle.smooth(img, radius, 1e-4)
+            stream = torch.cuda.Stream()
+            t = torch.from_numpy(img).cuda()
+            torch.cuda.synchronize()
+            for _ in range(4000):
+                q.smooth_device(t.data_ptr(), 20, 6, radius, 1e-4, stream=stream)
+            stream.synchronize()
+            t.copy_(torch.from_numpy(img))
+            torch.cuda.synchronize()
+            q.smooth_device(t.data_ptr(), 20, 6, radius, 1e-4, stream=stream)
+            stream.synchronize()
+            if not np.array_equal(t.cpu().numpy(), want):
+                failures.append(f"radius {radius}: not the oracle's image")
+        except Exception as e:
+            failures.append(f"radius {radius}: {e}")
+
+    threads = [threading.Thread(target=work, args=(r,)) for r in (60, 64)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures, failures
+
+
 def binned(img, k=8):
     h, w = img.shape
     h2, w2 = h // k * k, w // k * k
