@@ -77,12 +77,6 @@ __global__ void pool_kernel(PoolParams p) {
   p.perturbations[i] = make_float4(d.x, d.y, d.z, 0.0f);
 }
 
-__global__ void offsets_kernel(int* out, long long count, uint32_t seed, int heliostat, int pool) {
-  long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  out[i] = facet_offset(seed, (uint32_t)heliostat, (uint32_t)i, (uint32_t)pool);
-}
-
 // Facet offsets of every heliostat in one launch: element i of the buffer
 // belongs to heliostat h with seg[h] <= i < seg[h + 1].
 __global__ void offsets_all_kernel(int* out, const long long* seg, int heliostats, uint32_t seed, int pool) {
@@ -163,12 +157,6 @@ __global__ void xyz_to_float4_kernel(const float* xyz, float4* out, int n) {
 cudaError_t launch_pool(const PoolParams& p, cudaStream_t stream) {
   if (p.pool_size <= 0) return cudaSuccess;
   pool_kernel<<<(p.pool_size + 255) / 256, 256, 0, stream>>>(p);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_offsets(int* out, long long count, uint32_t seed, int heliostat, int pool, cudaStream_t stream) {
-  if (count <= 0) return cudaSuccess;
-  offsets_kernel<<<(unsigned)((count + 255) / 256), 256, 0, stream>>>(out, count, seed, heliostat, pool);
   return cudaGetLastError();
 }
 

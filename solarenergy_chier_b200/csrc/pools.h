@@ -43,7 +43,6 @@ struct PoolParams {
 };
 
 cudaError_t launch_pool(const PoolParams& p, cudaStream_t stream);
-cudaError_t launch_offsets(int* out, long long count, uint32_t seed, int heliostat, int pool, cudaStream_t stream);
 cudaError_t launch_xyz_to_float4(const float* xyz, float4* out, int n, cudaStream_t stream);
 // What the tracer needs to know of a sun-shape and a slope-error pool.
 struct PoolStats {
