@@ -156,7 +156,10 @@ int qmcrt_set_math_mode(qmcrt_scene* scene, int exact);
 /* Launch shapes of the production build (math mode 0), indexes 0..count-1:
  * threads per block, warp-chunk iterations (32 rays each) and whether the
  * launch is persistent (a grid of resident warps taking warp chunks from a
- * work counter, instead of one warp per chunk); shape 0 is the default.  No
+ * work counter, instead of one warp per chunk); shape 0 is the default, and
+ * the one that takes shorter chunks (8 or 16 iterations) and small receivers'
+ * spread images by itself: its flux launches below 64 M rays take fewer
+ * iterations than the table's, the others always theirs.  No
  * reference counterpart: the reference launches 512-thread blocks of one
  * ray each (Util/global_function.cuh:159-197).  Any array may be NULL; at
  * most 16 shapes. */
@@ -177,7 +180,8 @@ int qmcrt_set_light_range(qmcrt_scene* scene, int begin, int end);
  * (QuasiMonteCarloRayTracing/QuasiMonteCarloRayTracer.cpp:15-91): adds the
  * heliostat's flux into its receiver's image (images accumulate until
  * cleared) and its FP64 power into the per-heliostat total.  Asynchronous on
- * `stream`.  Invalid indexes fail as checkValidHeliostatIndex (:96-127) does. */
+ * `stream`.  Traces of one scene share the device copy of their list and the
+ * buffer of the power partials: order them, on one stream or by events.  Invalid indexes fail as checkValidHeliostatIndex (:96-127) does. */
 int qmcrt_trace_heliostat(qmcrt_scene* scene, int heliostat, void* stream);
 /* All listed heliostats in one launch (the loop of RayTracingPipeline.cpp:66-81). */
 int qmcrt_trace_heliostats(qmcrt_scene* scene, const int* heliostats, int n, void* stream);

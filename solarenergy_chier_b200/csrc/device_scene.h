@@ -125,8 +125,8 @@ __device__ __forceinline__ void begin_next() { asm volatile("griddepcontrol.laun
 // A launch whose blocks may be placed before the stream's previous kernel has
 // ended (the kernel calls wait_previous first); an ordinary launch while the
 // stream is being captured.  It hides a launch's 1.5 us, which counts between
-// a small trace and its power sum: 50 calls of 1.6 M rays 1,667 -> 1,516 us,
-// 24 M rays of 648 heliostats 476 -> 459.
+// a small trace and its power sum: it took 151 us off 50 calls of 1.6 M rays,
+// and 17 us of 476 off 24 M rays of 648 heliostats.
 template <class... P, class... A>
 cudaError_t launch_overlapped(void (*kernel)(P...), unsigned blocks, unsigned threads, cudaStream_t stream,
                               const A&... args) {
@@ -160,7 +160,7 @@ struct TraceParams {
   double* power;                  // FP64 per-slot power accumulators
   // flux and bilinear-deposit launches: when set, each warp chunk writes its
   // rays' FP64 energy sum to chunk_power[chunk - chunk_begin] and
-  // launch_power_reduce (power.cu) adds them per task into power, in a fixed
+  // launch_trace_end (power.cu) adds them per task into power, in a fixed
   // order with compensation; when NULL, one double atomic per chunk
   double* chunk_power;
   unsigned long long* diag;

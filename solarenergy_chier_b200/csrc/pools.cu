@@ -118,7 +118,7 @@ __global__ void trace_pools_kernel(const float4* in, const float4* pert, int n, 
 // pool as float bits (non-negative floats order like their bit patterns); +inf
 // when some direction has y <= 0.
 // Reduced per block: an atomic per warp made two words' 16,384 maxima the
-// kernel's time (12 us for 262,144 vectors, 4 so).
+// kernel's time (12 us for 262,144 vectors, 3 so).
 __global__ void __launch_bounds__(256) pool_stats_kernel(const float* dirs, const float* perts, int stride, int n,
                                                          PoolStats* out) {
   __shared__ unsigned found[3];  // bad, tan bits

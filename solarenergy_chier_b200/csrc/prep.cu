@@ -74,7 +74,7 @@ __global__ void prep_kernel(PrepInputs p) {
   atomicMax(it.top_key, height_key(isfinite(top) ? __float_as_int(top) : 0x7f800000));
 }
 
-// DevGrid::sub_free code of a block_candidates result: 1 nothing to hit,
+// DevGrid::sub_free code of a warp_candidates result: 1 nothing to hit,
 // k + 1 for k listed candidates, 0 walk (too many, or not enumerable).
 __device__ __forceinline__ int candidate_code(int k) {
   return k == 0 ? 1 : (k > 0 && k <= kMaxCandidates ? k + 1 : 0);

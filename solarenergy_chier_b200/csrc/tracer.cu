@@ -112,9 +112,8 @@ __device__ __forceinline__ int eps_order(float a, float b) {
 // Conservative slab test along one axis of a heliostat's padded box; ol and
 // dl are the ray origin (relative to the box centre) and direction along it.
 // The hardware reciprocal (1 ulp; infinite for dl = 0 and subnormal dl, where
-// the slab is then empty or the whole line) is one instruction against the
-// approximate division's five; the padding is far above its rounding.  The
-// 624-heliostat step, 85.5 -> 83.9 ms.
+// the slab is then empty or the whole line) in place of an approximate division;
+// the padding is far above its rounding.  The 624-heliostat step, 85.5 -> 83.9 ms.
 __device__ __forceinline__ void slab(float ol, float dl, float half, float& tn, float& tf) {
   float inv;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(dl));
