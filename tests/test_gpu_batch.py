@@ -211,6 +211,40 @@ def test_spread_images_and_large_ones(kind, pixel, tmp_path):
     np.testing.assert_allclose(out[1][1], out[0][1], rtol=1e-12, atol=0)
 
 
+@pytest.mark.parametrize("towers", [4, 5])
+def test_spread_images_of_as_many_receivers_as_there_are(towers, tmp_path):
+    """Scenes of four receivers have spread images, of five none: small
+    receivers side by side, traced one after another and all at once, give what
+    another launch shape's direct deposits do (L1 <= 1e-5, FP64 powers 1e-12)."""
+    f = synth.small_field(tmp_path, seed=1, groups=4, per_group=128, rows=2, cols=4)
+    lines = f.scene.read_text().splitlines()
+    first = lines.index("Recv\t0")
+    head, field = lines[:first], lines[first:]
+    out = [line.replace("ngrid\t1", f"ngrid\t{towers}") for line in head]
+    for k in range(towers):  # the same tower and field, 300 m further east
+        for line in field:
+            words = line.split()
+            if words and words[0] in ("pos", "helio"):
+                line = f"{words[0]}\t{float(words[1]) + 300.0 * k:.6f}\t{words[2]}\t{words[3]}"
+            out.append(line)
+    f.scene.write_text("\n".join(out) + "\n")
+    s = q.Scene(f.scene, f.config, device=0, seed=2)
+    assert s.num_receivers == towers and s.num_heliostats == 8 * towers
+    s.set_light_range(0, 32)  # 1.6 M rays a tower
+    images = []
+    for shape in (3, 0):
+        s.set_launch_shape(shape)
+        s.clear()
+        s.clear_power()
+        for k in range(towers):
+            s.trace(list(range(8 * k, 8 * k + 8)))
+        s.trace(list(range(8 * towers)))
+        images.append(([s.image(r).astype(np.float64) for r in range(towers)], s.power()[0]))
+    for a, b in zip(images[1][0], images[0][0]):
+        assert b.sum() > 0 and np.abs(a - b).sum() <= 1e-5 * b.sum()
+    np.testing.assert_allclose(images[1][1], images[0][1], rtol=1e-12, atol=0)
+
+
 def test_every_launch_shape_gives_the_same_result(fields, tmp_path):
     """The autotuner's candidates (launch shapes of the production build:
     block widths, warp chunks of 32, 64 or 128 iterations) change only how
